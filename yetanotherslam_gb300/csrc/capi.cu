@@ -236,6 +236,7 @@ YAS_API int yas_map_destroy(yas_map *m) {
 YAS_API int yas_map_reset(yas_map *m) {
     if (!m) return YAS_ERR_BAD_ARG;
     if (m->hibernated) return YAS_ERR_STATE;
+    m->edits++;
     launch_map_reset(map_view(m), m->stream);
     YAS_TRY_CUDA(cudaGetLastError());
     return YAS_OK;
@@ -275,6 +276,7 @@ YAS_API int yas_map_fuse_depth(yas_map *m, const float *depth, int width, int he
     YAS_TRY_CUDA(cudaMemcpyAsync(m->pose_dev, &pp, sizeof(pp), cudaMemcpyHostToDevice, m->stream));
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, width, height);
     MapDev v = map_view(m);
+    m->edits++;
     launch_allocate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, nullptr, m->stream);
     YAS_TRY_CUDA(cudaMemsetAsync(&m->hdr->n_visible, 0, sizeof(unsigned), m->stream));
     launch_visible(v, cam, m->pose_dev, nullptr, m->stream);
@@ -395,6 +397,7 @@ YAS_API int yas_map_import(yas_map *m, const int *coords, const float *sdf, cons
         cudaFree(dw);
         return YAS_ERR_OOM;
     }
+    m->edits++;
     int st = YAS_OK;
     if (cudaMemcpyAsync(dc, coords, (size_t)count * 12, cudaMemcpyHostToDevice, m->stream) != cudaSuccess ||
         cudaMemcpyAsync(ds, sdf, (size_t)count * 2048, cudaMemcpyHostToDevice, m->stream) != cudaSuccess ||
@@ -641,6 +644,7 @@ YAS_API int yas_map_load(yas_map *m, const char *path) {
         YAS_TRY_CUDA(cudaMemcpyAsync(m->voxels, vox.data(), vox.size(), cudaMemcpyHostToDevice, m->stream));
         YAS_TRY_CUDA(cudaMemcpyAsync(&m->hdr->n_alloc, &n, sizeof(unsigned), cudaMemcpyHostToDevice, m->stream));
         launch_rehash(map_view(m), n, m->stream);
+        m->edits++;
         YAS_TRY_CUDA(cudaGetLastError());
     }
     YAS_TRY(read_header(m));
@@ -715,6 +719,8 @@ static void swap_storage(yas_map *a, yas_map *b) {
     std::swap(a->hib_voxels, b->hib_voxels);
     std::swap(a->hib_visible, b->hib_visible);
     std::swap(a->hib_hdr, b->hib_hdr);
+    a->edits++;
+    b->edits++;
 }
 
 static int map_grow(yas_map *m, long long want_slots, long long want_blocks) {
@@ -822,6 +828,7 @@ YAS_API int yas_map_fuse_map(yas_map *dst, yas_map *src) {
     YAS_TRY(map_grow(dst, 2 * want_blocks, want_blocks));
     YAS_TRY_CUDA(cudaMemsetAsync(&dst->hdr->err_bits, 0, sizeof(unsigned), dst->stream));
     YAS_TRY_CUDA(cudaStreamSynchronize(src->stream));
+    dst->edits++;
     for (int attempt = 0;; ++attempt) {
         launch_fuse_alloc(map_view(dst), map_view(src), dst->cfg.voxel_format, T_src_dst, nsrc, dst->stream);
         YAS_TRY_CUDA(cudaGetLastError());
@@ -885,16 +892,7 @@ YAS_API int yas_raycaster_create(yas_raycaster **out, int width, int height, con
     rc->h = height;
     rc->cam = make_cam(K->fx, K->fy, K->cx, K->cy, width, height);
     rc->stream = (cudaStream_t)stream;
-    rc->rb.w = width;
-    rc->rb.h = height;
-    rc->rb.zw = (width + 7) / 8;
-    rc->rb.zh = (height + 7) / 8;
-    const size_t nz = (size_t)rc->rb.zw * rc->rb.zh;
-    rc->rb.fw = (width + (1 << kFineShift) - 1) >> kFineShift;
-    rc->rb.fh = (height + (1 << kFineShift) - 1) >> kFineShift;
-    if (cudaMalloc(&rc->rb.znear, nz * 4) != cudaSuccess || cudaMalloc(&rc->rb.zfar, nz * 4) != cudaSuccess ||
-        cudaMalloc(&rc->rb.queue, sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc(&rc->rb.fnear, (size_t)rc->rb.fw * rc->rb.fh * 4) != cudaSuccess ||
+    if (raycast_buffers_alloc(rc->rb, width, height) != YAS_OK ||
         cudaMalloc(&rc->vmap, (size_t)width * height * 16) != cudaSuccess ||
         cudaMalloc(&rc->depth_tmp, (size_t)width * height * 4) != cudaSuccess ||
         cudaMalloc(&rc->pose_dev, sizeof(PosePair)) != cudaSuccess) {
@@ -916,10 +914,7 @@ YAS_API int yas_raycaster_create(yas_raycaster **out, int width, int height, con
 YAS_API int yas_raycaster_destroy(yas_raycaster *rc) {
     if (!rc) return YAS_ERR_BAD_ARG;
     cudaStreamSynchronize(rc->stream);
-    cudaFree(rc->rb.znear);
-    cudaFree(rc->rb.zfar);
-    cudaFree(rc->rb.queue);
-    cudaFree(rc->rb.fnear);
+    raycast_buffers_free(rc->rb);
     cudaFree(rc->vmap);
     cudaFree(rc->depth_tmp);
     cudaFree(rc->pose_dev);

@@ -15,29 +15,92 @@
 // GB300 design: the z-range fill walks each visible block's footprint with
 // integer atomicMin/atomicMax on the float bit patterns (depths are positive,
 // so integer order equals float order) instead of CAS loops over split tiles;
-// the march caches the last block's pool index in registers, so consecutive
-// samples inside one 8^3 block cost one 4- or 8-byte load each.
+// a ray looks its blocks up in a dense grid of pool indices made for the view
+// and keeps the last one, so consecutive samples inside one 8^3 block cost one
+// 4- or 8-byte load each.  Per raycast (warm, events around the kernel; before:
+// hash lookups, image order, 32 rays a warp): 640x480, 5 mm F16 122 -> 79 us,
+// 1280x720, 4 mm F16 241 -> 166, 320x240, 8 mm F32 77 -> 50, 160x120, 1 cm F32
+// 72 -> 38.  What is left is instruction issue in large images (60% of the
+// slots; 20 of 32 lanes active) and the chain of the longest rays in small ones.
 // Deliberate differences: a missed ray writes w = -1 (the reference leaves w
 // stale on its early return, RayTraceEngine.cu:338-347); the 8 trilinear
 // corners are floor(p) + {0,1}^3 (the reference floors p + offset per corner).
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 
 #include "yas_internal.h"
 
 namespace yas {
 
-__global__ void zrange_reset_kernel(float *znear, float *zfar, int n, unsigned *n_render, unsigned *queue,
-                                    float *fnear, int nf) {
+// Block grid of a raycast: a cell for each of the kGridSide^3 blocks around the
+// middle of the view, which rays look their blocks up in instead of the hash
+// table.  A cell holds epoch << 24 | pool index; one of an earlier epoch is an
+// unallocated block, so cells are cleared only when the epoch wraps (every
+// 255th raycast).  Most lookups of a long ray are of unallocated blocks (59 of
+// 74 samples of the longest 2000 rays at 640x480, 5 mm): in the table each a
+// 64-bit hash and a read of a random line of 16-32 MB, here a few index
+// instructions and a line that neighbouring rays share.  (A bit per block in
+// front of the cells, kept by the ray per 4x4x4 blocks, saved reads but cost
+// more in instructions: 174 against 161 us at 1280x720, 4 mm.)  Blocks outside
+// the grid, and those whose index does not fit 24 bits (kGridAsk), are looked
+// up in the table.
+// info: first block x, y, z; epoch; epoch of the next raycast.
+constexpr unsigned kGridAsk = 0xffffffu;
+
+__device__ __forceinline__ int grid_cell(int x, int y, int z) { return (z * kGridSide + y) * kGridSide + x; }
+__device__ __forceinline__ bool grid_holds(int x, int y, int z) {
+    return max(max((unsigned)x, (unsigned)y), (unsigned)z) < (unsigned)kGridSide;
+}
+
+// Opens an epoch: the grid is centred half way along the depth range, at most
+// 64 blocks ahead of the camera.  (grid_fill, the next kernel, writes info[4].)
+__device__ __forceinline__ void grid_begin(const MapDev &m, const PosePair *P, const BlockGrid &g) {
+    const int next = g.info[4], epoch = next < 1 || next > 255 ? 1 : next;
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (epoch == 1)
+        for (int i = i0; i < kGridCells / 4; i += stride)
+            reinterpret_cast<uint4 *>(g.cells)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (i0 == 0) {
+        const float side = m.voxel_size * (float)kBlockSide;
+        const float3 c = rigid_fast(P->T, 0.0f, 0.0f, fminf(0.5f * m.depth_max, 64.0f * side));
+        const float lim = 1.0e8f;  // far outside the key range
+        g.info[0] = (int)floorf(fmaxf(-lim, fminf(lim, c.x / side))) - kGridSide / 2;
+        g.info[1] = (int)floorf(fmaxf(-lim, fminf(lim, c.y / side))) - kGridSide / 2;
+        g.info[2] = (int)floorf(fmaxf(-lim, fminf(lim, c.z / side))) - kGridSide / 2;
+        g.info[3] = epoch;
+    }
+}
+
+__device__ __forceinline__ void grid_fill(const MapDev &m, const BlockGrid &g) {
+    const int ox = g.info[0], oy = g.info[1], oz = g.info[2];
+    const unsigned epoch = (unsigned)g.info[3] << 24, n = num_blocks(m);
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        int x, y, z;
+        unpack_key(m.block_keys[i], x, y, z);
+        x -= ox, y -= oy, z -= oz;
+        if (grid_holds(x, y, z)) g.cells[grid_cell(x, y, z)] = epoch | min(i, kGridAsk);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) g.info[4] = g.info[3] + 1;
+}
+
+__global__ void zrange_reset_kernel(MapDev m, const PosePair *P, float *znear, float *zfar, int n, unsigned *queue,
+                                    float *fnear, int nf, BlockGrid g) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         znear[i] = 100.0f;
         zfar[i] = 0.0f;
     }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nf; i += gridDim.x * blockDim.x) fnear[i] = 100.0f;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *n_render = 0;
-        *queue = 0u;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *queue = 0u;
+    grid_begin(m, P, g);
+}
+
+__global__ void __launch_bounds__(256) grid_begin_kernel(MapDev m, const PosePair *P, BlockGrid g) {
+    grid_begin(m, P, g);
+}
+
+__global__ void __launch_bounds__(256) grid_fill_kernel(MapDev m, BlockGrid g) {
+    grid_fill(m, g);
 }
 
 __device__ __forceinline__ int clamp_floor(float v) {
@@ -53,8 +116,10 @@ __device__ __forceinline__ int clamp_ceil(float v) {
 
 __global__ void __launch_bounds__(128) zrange_fill_kernel(MapDev m, Cam cam, const PosePair *P,
                                                           float *znear, float *zfar, int zw, int zh,
-                                                          const int *skip, float *fnear, int fw, int fh) {
+                                                          const int *skip, float *fnear, int fw, int fh,
+                                                          BlockGrid g) {
     if (skip && *skip) return;
+    grid_fill(m, g);
     const unsigned nvis = *(volatile unsigned *)&m.hdr->n_visible;
     const Rigid32 Tinv = P->Tinv;
     const float scale = m.voxel_size * 8.0f;
@@ -114,114 +179,128 @@ __global__ void __launch_bounds__(128) zrange_fill_kernel(MapDev m, Cam cam, con
                 atomicMin(reinterpret_cast<int *>(znear) + y * zw + x, inear);
                 atomicMax(reinterpret_cast<int *>(zfar) + y * zw + x, ifar);
             }
-        unsigned tiles = (unsigned)(((lrx - ulx + 16) / 16) * ((lry - uly + 16) / 16));
-        atomicAdd(&m.hdr->n_render, tiles);
     }
+}
+
+int raycast_buffers_alloc(RaycastBuffers &rb, int width, int height) {
+    rb.w = width;
+    rb.h = height;
+    rb.zw = (width + 7) / 8;
+    rb.zh = (height + 7) / 8;
+    rb.fw = (width + (1 << kFineShift) - 1) >> kFineShift;
+    rb.fh = (height + (1 << kFineShift) - 1) >> kFineShift;
+    const size_t nz = (size_t)rb.zw * rb.zh;
+    if (cudaMalloc(&rb.znear, nz * 4) != cudaSuccess || cudaMalloc(&rb.zfar, nz * 4) != cudaSuccess ||
+        cudaMalloc(&rb.queue, sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&rb.fnear, (size_t)rb.fw * rb.fh * 4) != cudaSuccess ||
+        cudaMalloc(&rb.grid.cells, kGridCells * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&rb.grid.info, 5 * sizeof(int)) != cudaSuccess) {
+        cudaGetLastError();
+        return YAS_ERR_OOM;
+    }
+    // no epoch yet: the first raycast clears the cells.  The fill runs on the
+    // legacy stream, which the raycaster's non-blocking stream does not wait for
+    if (cudaMemset(rb.grid.info, 0, 5 * sizeof(int)) != cudaSuccess ||
+        cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)
+        return YAS_ERR_CUDA;
+    return YAS_OK;
+}
+
+void raycast_buffers_free(RaycastBuffers &rb) {
+    cudaFree(rb.znear);
+    cudaFree(rb.zfar);
+    cudaFree(rb.queue);
+    cudaFree(rb.fnear);
+    cudaFree(rb.grid.cells);
+    cudaFree(rb.grid.info);
+    rb = RaycastBuffers{};
 }
 
 void launch_zrange(const MapDev &m, const Cam &cam, const PosePair *P, RaycastBuffers &rb,
                    const int *skip, cudaStream_t s) {
     const int n = rb.zw * rb.zh, nf = rb.fw * rb.fh;
-    zrange_reset_kernel<<<(std::max(n, nf) + 255) / 256, 256, 0, s>>>(rb.znear, rb.zfar, n, &m.hdr->n_render,
-                                                                      rb.queue, rb.fnear, nf);
+    zrange_reset_kernel<<<(std::max(n, nf) + 255) / 256, 256, 0, s>>>(m, P, rb.znear, rb.zfar, n, rb.queue, rb.fnear,
+                                                                      nf, rb.grid);
     zrange_fill_kernel<<<kSMs * 2, 128, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, rb.zh, skip, rb.fnear, rb.fw,
-                                               rb.fh);
+                                               rb.fh, rb.grid);
 }
 
-// Block-pointer cache of one ray.
-template <int FMT>
-struct VoxelReader {
-    typedef VoxelIO<FMT> IO;
-    const MapDev &m;
-    const typename IO::T *vox;
-    unsigned long long ckey;
-    int cptr;
-    __device__ __forceinline__ VoxelReader(const MapDev &mm)
-        : m(mm), vox(static_cast<const typename IO::T *>(mm.voxels)), ckey(kEmptyKey), cptr(-1) {}
+void launch_block_grid(const MapDev &m, const PosePair *P, const RaycastBuffers &rb, cudaStream_t s) {
+    grid_begin_kernel<<<kSMs, 256, 0, s>>>(m, P, rb.grid);
+    grid_fill_kernel<<<kSMs, 256, 0, s>>>(m, rb.grid);
+}
 
-    // sdf of voxel (vx,vy,vz); valid = observed (weight != 0)
-    __device__ __forceinline__ float read(int vx, int vy, int vz, bool &valid) {
-        int bx = vx >> 3, by = vy >> 3, bz = vz >> 3;
-        unsigned long long k = pack_key(bx, by, bz);
-        if (k != ckey) {
-            ckey = k;
-            cptr = coord_in_range(bx, by, bz) ? find_block(m, k) : -1;
+// Reads of one ray.
+template <int FMT>
+struct RayReader {
+    typedef VoxelIO<FMT> IO;
+    typedef typename IO::T V;
+    const MapDev &m;
+    const BlockGrid &g;
+    const V *vox;
+    int ox, oy, oz;  // the grid's first block
+    unsigned epoch;  // and its epoch << 24
+
+    __device__ __forceinline__ RayReader(const MapDev &mm, const BlockGrid &gg)
+        : m(mm), g(gg), vox(static_cast<const V *>(mm.voxels)), ox(__ldg(gg.info)), oy(__ldg(gg.info + 1)),
+          oz(__ldg(gg.info + 2)), epoch((unsigned)__ldg(gg.info + 3) << 24) {}
+
+    // Pool index of block (x, y, z), or -1.
+    __device__ __forceinline__ int lookup(int x, int y, int z) const {
+        const int gx = x - ox, gy = y - oy, gz = z - oz;
+        if (grid_holds(gx, gy, gz)) {
+            const unsigned w = __ldg(g.cells + grid_cell(gx, gy, gz)) - epoch;  // below 2^24 in this epoch only
+            if (w != kGridAsk) return w < kGridAsk ? (int)w : -1;
         }
-        if (cptr < 0) {
-            valid = false;
-            return 1.0f;
-        }
-        typename IO::T v = __ldg(vox + (size_t)cptr * kBlockVoxels + ((vz & 7) << 6) + ((vy & 7) << 3) + (vx & 7));
-        if (IO::wt(v) == 0) {
-            valid = false;
-            return 1.0f;
-        }
-        valid = true;
-        return IO::sdf(v);
+        return find_block_xyz(m, x, y, z);
     }
-    __device__ __forceinline__ float read_nearest(float3 p, bool &valid) {
-        return read((int)floorf(p.x), (int)floorf(p.y), (int)floorf(p.z), valid);
+    // voxel (vx,vy,vz) of pool block b
+    __device__ __forceinline__ V at(int b, int vx, int vy, int vz) const {
+        return __ldg(vox + (size_t)b * kBlockVoxels + ((vz & 7) << 6) + ((vy & 7) << 3) + (vx & 7));
     }
-    // Trilinear sample with the reference's lerp order (RayTraceEngine.cu:297-329).
-    __device__ __forceinline__ float corner(typename IO::T v, bool &ok) {
+    // sdf of a voxel word; ok is cleared when it is unobserved (weight 0)
+    __device__ __forceinline__ float value(V v, bool &ok) const {
         if (IO::wt(v) == 0) {
             ok = false;
             return 1.0f;
         }
         return IO::sdf(v);
     }
-    __device__ __forceinline__ float read_interp(float3 p, bool &valid) {
-        float fx = floorf(p.x), fy = floorf(p.y), fz = floorf(p.z);
-        int x0 = (int)fx, y0 = (int)fy, z0 = (int)fz;
-        float ax = p.x - fx, ay = p.y - fy, az = p.z - fz;
-        if ((x0 & 7) != 7 && (y0 & 7) != 7 && (z0 & 7) != 7) {
-            // the 2x2x2 cell lies in one block: eight independent loads at
-            // fixed offsets from one base, same lerp order as the general path
-            int bx = x0 >> 3, by = y0 >> 3, bz = z0 >> 3;
-            unsigned long long k = pack_key(bx, by, bz);
-            if (k != ckey) {
-                ckey = k;
-                cptr = coord_in_range(bx, by, bz) ? find_block(m, k) : -1;
-            }
-            if (cptr < 0) {
-                valid = false;
-                return 1.0f;
-            }
-            const typename IO::T *b =
-                vox + (size_t)cptr * kBlockVoxels + ((z0 & 7) << 6) + ((y0 & 7) << 3) + (x0 & 7);
-            const typename IO::T q0 = __ldg(b), q1 = __ldg(b + 1), q2 = __ldg(b + 8), q3 = __ldg(b + 9);
-            const typename IO::T q4 = __ldg(b + 64), q5 = __ldg(b + 65), q6 = __ldg(b + 72), q7 = __ldg(b + 73);
-            bool ok = true;
-            const float s000 = corner(q0, ok), s100 = corner(q1, ok), s010 = corner(q2, ok), s110 = corner(q3, ok);
-            const float s001 = corner(q4, ok), s101 = corner(q5, ok), s011 = corner(q6, ok), s111 = corner(q7, ok);
-            float r0 = (1.0f - ax) * s000 + ax * s100;
-            float r1 = (1.0f - ax) * s010 + ax * s110;
-            const float r2 = (1.0f - ay) * r0 + ay * r1;
-            r0 = (1.0f - ax) * s001 + ax * s101;
-            r1 = (1.0f - ax) * s011 + ax * s111;
-            const float r3 = (1.0f - ay) * r0 + ay * r1;
-            valid = ok;
-            return (1.0f - az) * r2 + az * r3;
+    // Trilinear sample at p, whose block (bx, by, bz) has pool index b, with the
+    // reference's lerp order (RayTraceEngine.cu:297-329).  A third of the 2x2x2
+    // cells straddle a block face: their lanes look the neighbours up (1, 3 or
+    // 7 of them, the submasks d of the straddled axes; corner c lies in
+    // neighbour c & across), then every lane reads its eight corners.
+    __device__ __forceinline__ float interp(float3 p, int bx, int by, int bz, int b, bool &valid) const {
+        const float fx = floorf(p.x), fy = floorf(p.y), fz = floorf(p.z);
+        const int x0 = (int)fx, y0 = (int)fy, z0 = (int)fz;
+        const float ax = p.x - fx, ay = p.y - fy, az = p.z - fz;
+        const unsigned across = ((x0 & 7) == 7 ? 1u : 0u) | ((y0 & 7) == 7 ? 2u : 0u) | ((z0 & 7) == 7 ? 4u : 0u);
+        int q[8];  // pool index of each corner's block
+#pragma unroll
+        for (int c = 0; c < 8; ++c) q[c] = b;
+        for (unsigned d = across; d != 0u; d = (d - 1u) & across) {
+            const int e = lookup(bx + (int)(d & 1u), by + (int)((d >> 1) & 1u), bz + (int)(d >> 2));
+#pragma unroll
+            for (unsigned c = 1u; c < 8u; ++c) q[c] = (c & across) == d ? e : q[c];
         }
-        bool v0, v1, ok = true;
-        float s0 = read(x0, y0, z0, v0);
-        float s1 = read(x0 + 1, y0, z0, v1);
-        ok = v0 && v1;
-        float r0 = (1.0f - ax) * s0 + ax * s1;
-        s0 = read(x0, y0 + 1, z0, v0);
-        s1 = read(x0 + 1, y0 + 1, z0, v1);
-        ok = ok && v0 && v1;
-        float r1 = (1.0f - ax) * s0 + ax * s1;
-        float r2 = (1.0f - ay) * r0 + ay * r1;
-        s0 = read(x0, y0, z0 + 1, v0);
-        s1 = read(x0 + 1, y0, z0 + 1, v1);
-        ok = ok && v0 && v1;
-        r0 = (1.0f - ax) * s0 + ax * s1;
-        s0 = read(x0, y0 + 1, z0 + 1, v0);
-        s1 = read(x0 + 1, y0 + 1, z0 + 1, v1);
-        ok = ok && v0 && v1;
-        r1 = (1.0f - ax) * s0 + ax * s1;
-        float r3 = (1.0f - ay) * r0 + ay * r1;
+        const int xo[2] = {x0 & 7, (x0 + 1) & 7}, yo[2] = {(y0 & 7) << 3, ((y0 + 1) & 7) << 3};
+        const int zo[2] = {(z0 & 7) << 6, ((z0 + 1) & 7) << 6};
+        V v[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+            v[c] = q[c] >= 0 ? __ldg(vox + (size_t)q[c] * kBlockVoxels + (zo[c >> 2] + yo[(c >> 1) & 1] + xo[c & 1]))
+                             : IO::make(1.0f, 0);
+        bool ok = true;
+        float s[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) s[c] = value(v[c], ok);
+        float r0 = (1.0f - ax) * s[0] + ax * s[1];
+        float r1 = (1.0f - ax) * s[2] + ax * s[3];
+        const float r2 = (1.0f - ay) * r0 + ay * r1;
+        r0 = (1.0f - ax) * s[4] + ax * s[5];
+        r1 = (1.0f - ax) * s[6] + ax * s[7];
+        const float r3 = (1.0f - ay) * r0 + ay * r1;
         valid = ok;
         return (1.0f - az) * r2 + az * r3;
     }
@@ -231,8 +310,6 @@ struct VoxelReader {
 struct RayState {
     float3 r, dir, idir;
     float dist_s, dist_e, sdf;
-    bool valid;
-    unsigned long long skipped;
 };
 
 // Ray of pixel (x, y) between the tile's z-range bounds zn..zf; false when the
@@ -258,11 +335,9 @@ __device__ __forceinline__ bool ray_setup(const Cam &cam, const Rigid32 &T, floa
     if (dn > 0.0f) dir = make_float3(dir.x / dn, dir.y / dn, dir.z / dn);
     R.r = s;
     R.dir = dir;
-    R.idir = make_float3(dir.x != 0.0f ? 1.0f / dir.x : 0.0f, dir.y != 0.0f ? 1.0f / dir.y : 0.0f,
-                         dir.z != 0.0f ? 1.0f / dir.z : 0.0f);
-    R.skipped = kEmptyKey;
+    R.idir = make_float3(dir.x != 0.0f ? -1.0f / fabsf(dir.x) : 1.0f, dir.y != 0.0f ? -1.0f / fabsf(dir.y) : 1.0f,
+                         dir.z != 0.0f ? -1.0f / fabsf(dir.z) : 1.0f);
     R.sdf = 1.0f;
-    R.valid = false;
     if (zfine > zn) {
         const float k = sqrtf(ux * ux + uy * uy + 1.0f) * vsinv;  // voxels of ray per metre of depth
         const float n = floorf(fminf(zfine * k, R.dist_e) - R.dist_s) - 2.0f;
@@ -274,65 +349,76 @@ __device__ __forceinline__ bool ray_setup(const Cam &cam, const Rigid32 &T, floa
     return true;
 }
 
-// One iteration of the march loop; true once the ray is finished (a sample
-// with sdf <= 0, or the end of its range).
+// One axis of a ray in an unallocated block whose lower face is at x0.  `face`
+// is the face that the ray leaves through (1e30 for a ray parallel to the
+// axis: none); the result is the steps to the first sample at or past it (the
+// upper face is outside the block, the lower one inside).  idir is -1 / dir
+// for a rising ray, 1 / dir for a falling one, 1 for a parallel one.
+__device__ __forceinline__ float exit_steps(float x0, float r, float dir, float idir, float &face) {
+    const bool falls = dir < 0.0f;
+    face = x0 + (falls ? 0.0f : (dir > 0.0f ? 8.0f : 1e30f));
+    const float t = floorf((face - r) * idir);
+    return falls ? t + 1.0f : (dir > 0.0f ? -t : 1e30f);
+}
+// p is outside the block on that axis (it came from inside along dir).
+__device__ __forceinline__ bool past(float p, float dir, float face) { return (p >= face) != (dir < 0.0f); }
+
+// Samples to the first one past the unallocated block that holds the sample at
+// R.r (its lower corner at x0, y0, z0): every sample until the ray leaves the
+// block reads "unobserved" and advances one voxel, so they are taken in one
+// move.  k = steps to the first sample outside on the earliest exit axis.  When
+// sample k - 1 (computed as the move computes it) is still in the block and
+// sample k is not, the move goes straight to sample k; otherwise (k rounded
+// the wrong way) it keeps two samples as margin, at least one step.
+__device__ __forceinline__ float empty_steps(const RayState &R, float x0, float y0, float z0) {
+    float fx, fy, fz;
+    const float kx = exit_steps(x0, R.r.x, R.dir.x, R.idir.x, fx), ky = exit_steps(y0, R.r.y, R.dir.y, R.idir.y, fy);
+    const float kz = exit_steps(z0, R.r.z, R.dir.z, R.idir.z, fz);
+    const float k = fminf(fminf(kx, ky), kz), a = k - 1.0f;
+    const bool in = !(past(R.r.x + a * R.dir.x, R.dir.x, fx) || past(R.r.y + a * R.dir.y, R.dir.y, fy) ||
+                      past(R.r.z + a * R.dir.z, R.dir.z, fz));
+    const bool out = past(R.r.x + k * R.dir.x, R.dir.x, fx) || past(R.r.y + k * R.dir.y, R.dir.y, fy) ||
+                     past(R.r.z + k * R.dir.z, R.dir.z, fz);
+    const float n = k >= 1.0f && k < 1e29f && in && out ? k : k - 2.0f;
+    return fmaxf(fminf(n, ceilf(R.dist_e - R.dist_s)), 1.0f);
+}
+
+// The march loop, to a sample with sdf <= 0 or the end of the ray's range.
 template <int FMT>
-__device__ __forceinline__ bool ray_step(VoxelReader<FMT> &rd, float rstep, RayState &R) {
-    if (!(R.dist_s < R.dist_e)) return true;
-    R.sdf = rd.read_nearest(R.r, R.valid);
-    if (rd.cptr < 0 && rd.ckey != R.skipped) {
-        // Unallocated block: every sample until the ray leaves it reads
-        // "unobserved" and advances one voxel, so those samples are skipped in
-        // one move.  k = steps to the first sample outside the block on the
-        // earliest exit axis.  When sample k - 1 (computed as the jump computes
-        // it) is still in the block and sample k is not, the ray jumps straight
-        // to sample k; otherwise (k rounded the wrong way) it keeps two samples
-        // as margin and evaluates the last ones inside the block normally.
-        R.skipped = rd.ckey;
-        const float bx0 = floorf(floorf(R.r.x) * 0.125f) * 8.0f;
-        const float by0 = floorf(floorf(R.r.y) * 0.125f) * 8.0f;
-        const float bz0 = floorf(floorf(R.r.z) * 0.125f) * 8.0f;
-        const float kx = R.dir.x > 0.0f ? ceilf((bx0 + 8.0f - R.r.x) * R.idir.x)
-                                        : (R.dir.x < 0.0f ? floorf((bx0 - R.r.x) * R.idir.x) + 1.0f : 1e30f);
-        const float ky = R.dir.y > 0.0f ? ceilf((by0 + 8.0f - R.r.y) * R.idir.y)
-                                        : (R.dir.y < 0.0f ? floorf((by0 - R.r.y) * R.idir.y) + 1.0f : 1e30f);
-        const float kz = R.dir.z > 0.0f ? ceilf((bz0 + 8.0f - R.r.z) * R.idir.z)
-                                        : (R.dir.z < 0.0f ? floorf((bz0 - R.r.z) * R.idir.z) + 1.0f : 1e30f);
-        const float k = fminf(fminf(kx, ky), kz);
-        float n = k - 2.0f;
-        if (k >= 1.0f && k < 1e29f) {
-            const float a = k - 1.0f;
-            const float3 pin = make_float3(R.r.x + a * R.dir.x, R.r.y + a * R.dir.y, R.r.z + a * R.dir.z);
-            const float3 pout = make_float3(R.r.x + k * R.dir.x, R.r.y + k * R.dir.y, R.r.z + k * R.dir.z);
-            const unsigned long long kin =
-                pack_key((int)floorf(pin.x) >> 3, (int)floorf(pin.y) >> 3, (int)floorf(pin.z) >> 3);
-            const unsigned long long kout =
-                pack_key((int)floorf(pout.x) >> 3, (int)floorf(pout.y) >> 3, (int)floorf(pout.z) >> 3);
-            if (kin == rd.ckey && kout != rd.ckey) n = k;
+__device__ __forceinline__ void ray_march(const RayReader<FMT> &rd, float rstep, RayState &R) {
+    int bx = INT_MIN, by = 0, bz = 0;  // the block of the sample at R.r
+    int cptr = -1;                     // its pool index (-1: unallocated)
+    bool jumped = false;               // the ray has taken its jump out of that (unallocated) block
+    while (R.dist_s < R.dist_e) {
+        float n = 1.0f;
+        const int vx = (int)floorf(R.r.x), vy = (int)floorf(R.r.y), vz = (int)floorf(R.r.z);
+        const int x = vx >> 3, y = vy >> 3, z = vz >> 3;
+        if (x != bx || y != by || z != bz) {
+            bx = x, by = y, bz = z;
+            jumped = false;
+            cptr = rd.lookup(x, y, z);
         }
-        n = fminf(n, ceilf(R.dist_e - R.dist_s));
-        if (n >= 1.0f) {
-            R.r.x += n * R.dir.x;
-            R.r.y += n * R.dir.y;
-            R.r.z += n * R.dir.z;
-            R.dist_s += n;
-            return false;
+        if (cptr < 0) {
+            if (!jumped) n = empty_steps(R, (float)(vx & ~7), (float)(vy & ~7), (float)(vz & ~7));
+            jumped = true;
+        } else {
+            bool valid = true;
+            R.sdf = rd.value(rd.at(cptr, vx, vy, vz), valid);
+            if (R.sdf <= 0.5f && R.sdf >= -0.5f) R.sdf = rd.interp(R.r, bx, by, bz, cptr, valid);
+            if (R.sdf <= 0.0f) return;
+            if (valid) n = fmaxf(R.sdf * rstep, 1.0f);
         }
+        R.r.x += n * R.dir.x;
+        R.r.y += n * R.dir.y;
+        R.r.z += n * R.dir.z;
+        R.dist_s += n;
     }
-    if (R.sdf <= 0.5f && R.sdf >= -0.5f) R.sdf = rd.read_interp(R.r, R.valid);
-    if (R.sdf <= 0.0f) return true;
-    const float step = R.valid ? fmaxf(R.sdf * rstep, 1.0f) : 1.0f;
-    R.r.x += step * R.dir.x;
-    R.r.y += step * R.dir.y;
-    R.r.z += step * R.dir.z;
-    R.dist_s += step;
-    return false;
 }
 
 // Vertex of a finished ray: a hit takes two interpolated correction steps
 // and is returned in camera coordinates (w = 1); a miss is NaN with w = -1.
 template <int FMT>
-__device__ __forceinline__ float4 ray_finish(VoxelReader<FMT> &rd, float rstep, float vsinv, const Rigid32 &Ti,
+__device__ __forceinline__ float4 ray_finish(const RayReader<FMT> &rd, float rstep, float vsinv, const Rigid32 &Ti,
                                              RayState &R) {
     float4 out = make_float4(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff), __int_as_float(0x7fffffff),
                              -1.0f);
@@ -341,12 +427,15 @@ __device__ __forceinline__ float4 ray_finish(VoxelReader<FMT> &rd, float rstep, 
         R.r.x += step * R.dir.x;
         R.r.y += step * R.dir.y;
         R.r.z += step * R.dir.z;
-        R.sdf = rd.read_interp(R.r, R.valid);
+        const int x = (int)floorf(R.r.x) >> 3, y = (int)floorf(R.r.y) >> 3, z = (int)floorf(R.r.z) >> 3;
+        const int b = rd.lookup(x, y, z);
+        bool valid = false;
+        R.sdf = b >= 0 ? rd.interp(R.r, x, y, z, b, valid) : 1.0f;
         step = R.sdf * rstep;
         R.r.x += step * R.dir.x;
         R.r.y += step * R.dir.y;
         R.r.z += step * R.dir.z;
-        if (R.valid) {
+        if (valid) {
             const float3 w = make_float3(R.r.x / vsinv, R.r.y / vsinv, R.r.z / vsinv);
             const float3 c = rigid_fast(Ti, w.x, w.y, w.z);
             out = make_float4(c.x, c.y, c.z, 1.0f);
@@ -355,33 +444,56 @@ __device__ __forceinline__ float4 ray_finish(VoxelReader<FMT> &rd, float rstep, 
     return out;
 }
 
-// One thread per pixel; each warp a compact 8x4 tile, so its rays travel
-// similar depths; the CTA's WX x WY warp tiles cover 8WX x 4WY pixels.
-template <int FMT, int WX, int WY>
+// The pixel (x, y) of each lane of a warp (outside the image: none).  `turn` 0:
+// only if the warp has a long ray, 1: only if it has none, -1: always.  A ray
+// is long when more than kLongBlocks blocks lie between the first visible
+// block in front of its pixels and the far bound of its tile.  Each tile is
+// launched for both turns, the long ones in the first half of the grid: a warp
+// of long rays takes most of the march's time wherever it starts (640x480, 5
+// mm: 97 us in image order, 85 with the long ones first; 4 or 32 blocks: 92
+// and 96).
+constexpr float kLongBlocks = 8.0f;
+template <int FMT>
+__device__ __forceinline__ void march_pixel(const MapDev &m, const Cam &cam, const PosePair *P,
+                                            const float *__restrict__ znear, const float *__restrict__ zfar, int zw,
+                                            float4 *vmap, int vpitch, bool skipped, const float *__restrict__ fnear,
+                                            int fw, const BlockGrid &g, int x, int y, int turn) {
+    const float vsinv = 1.0f / m.voxel_size;
+    const float rstep = m.trunc / m.voxel_size;
+    const bool inside = x < cam.w && y < cam.h;
+    RayState R;
+    R.sdf = 1.0f;
+    float zn = 0.0f, zf = 0.0f, zfine = 0.0f;
+    if (inside && !skipped) {
+        zn = __ldg(znear + (y >> 3) * zw + (x >> 3));
+        zf = __ldg(zfar + (y >> 3) * zw + (x >> 3));
+        zfine = __ldg(fnear + (y >> kFineShift) * fw + (x >> kFineShift));
+    }
+    if (turn >= 0) {
+        const bool far = zf - fmaxf(zn, zfine) > kLongBlocks * (float)kBlockSide * m.voxel_size;
+        if ((int)!__any_sync(0xffffffffu, far) != turn) return;
+    }
+    const bool live = inside && !skipped && ray_setup(cam, P->T, vsinv, zn, zf, zfine, x, y, R);
+    const RayReader<FMT> rd(m, g);
+    if (live) ray_march(rd, rstep, R);
+    if (inside) vmap[(size_t)y * vpitch + x] = ray_finish(rd, rstep, vsinv, P->Tinv, R);
+}
+
+// Each warp a compact tile of RAYS pixels (32: 8x4, 16: 4x4, 8: 4x2), so its
+// rays travel similar depths; a CTA is WX x WY warp tiles.  Warps of fewer rays
+// leave lanes idle and run more instructions in all, but each warp less: the
+// lanes of a warp that jump, look up and sample take turns.
+template <int FMT, int WX, int WY, int RAYS>
 __global__ void __launch_bounds__(32 * WX * WY) march_kernel(MapDev m, Cam cam, const PosePair *P,
                                                              const float *__restrict__ znear,
                                                              const float *__restrict__ zfar, int zw, float4 *vmap,
                                                              int vpitch, const int *skip,
-                                                             const float *__restrict__ fnear, int fw) {
+                                                             const float *__restrict__ fnear, int fw, BlockGrid g) {
+    constexpr int TX = RAYS == 32 ? 8 : 4, TY = RAYS / TX;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int x = blockIdx.x * (8 * WX) + (warp % WX) * 8 + (lane & 7);
-    const int y = blockIdx.y * (4 * WY) + (warp / WX) * 4 + (lane >> 3);
-    if (x >= cam.w || y >= cam.h) return;
-    float4 out = make_float4(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff), __int_as_float(0x7fffffff),
-                             -1.0f);
-    if (!(skip && *skip)) {
-        const float vsinv = 1.0f / m.voxel_size;
-        const float rstep = m.trunc / m.voxel_size;
-        RayState R;
-        if (ray_setup(cam, P->T, vsinv, __ldg(znear + (y >> 3) * zw + (x >> 3)), __ldg(zfar + (y >> 3) * zw + (x >> 3)),
-                      __ldg(fnear + (y >> kFineShift) * fw + (x >> kFineShift)), x, y, R)) {
-            VoxelReader<FMT> rd(m);
-            while (!ray_step(rd, rstep, R)) {
-            }
-            out = ray_finish(rd, rstep, vsinv, P->Tinv, R);
-        }
-    }
-    vmap[(size_t)y * vpitch + x] = out;
+    const int x = lane < RAYS ? (blockIdx.x * WX + warp % WX) * TX + lane % TX : INT_MAX;
+    const int y = (blockIdx.y * WY + warp / WX) * TY + lane / TX;
+    march_pixel<FMT>(m, cam, P, znear, zfar, zw, vmap, vpitch, skip && *skip, fnear, fw, g, x, y, (int)blockIdx.z);
 }
 
 // Persistent march: resident warps take 8x4-pixel tiles from a queue (one
@@ -393,60 +505,19 @@ template <int FMT>
 __global__ void __launch_bounds__(128) march_persistent_kernel(MapDev m, Cam cam, const PosePair *P,
                                                                const float *__restrict__ znear,
                                                                const float *__restrict__ zfar, int zw, float4 *vmap,
-                                                               int vpitch, const int *skip, unsigned *queue,
-                                                               unsigned total, const float *__restrict__ fnear,
-                                                               int fw) {
-    const unsigned lane = lane_id();
-    const int tiles_x = (cam.w + 7) >> 3;
-    const float4 miss = make_float4(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff),
-                                    __int_as_float(0x7fffffff), -1.0f);
-    if (skip && *skip) {
-        for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
-            const int t = (int)(p >> 5), l = (int)(p & 31u);
-            const int x = (t % tiles_x) * 8 + (l & 7), y = (t / tiles_x) * 4 + (l >> 3);
-            if (x < cam.w && y < cam.h) vmap[(size_t)y * vpitch + x] = miss;
-        }
-        return;
-    }
-    const float vsinv = 1.0f / m.voxel_size;
-    const float rstep = m.trunc / m.voxel_size;
-    VoxelReader<FMT> rd(m);
-    RayState R;
-    bool active = false, drained = false;
-    int x = 0, y = 0;
+                                                               int vpitch, const int *skip,
+                                                               const float *__restrict__ fnear, int fw,
+                                                               BlockGrid g, unsigned *queue,
+                                                               unsigned tiles) {
+    const int lane = (int)lane_id(), tiles_x = (cam.w + 7) >> 3;
+    const bool skipped = skip && *skip;
     for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, !active);
-        if (!drained && idle == 0xffffffffu) {
-            const int leader = __ffs(idle) - 1;
-            unsigned base = 0u;
-            if ((int)lane == leader) base = atomicAdd(queue, (unsigned)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base + (unsigned)__popc(idle) >= total) drained = true;
-            if (!active) {
-                const unsigned p = base + (unsigned)__popc(idle & ((1u << lane) - 1u));
-                if (p < total) {
-                    const int t = (int)(p >> 5), l = (int)(p & 31u);
-                    x = (t % tiles_x) * 8 + (l & 7);
-                    y = (t / tiles_x) * 4 + (l >> 3);
-                    if (x < cam.w && y < cam.h) {
-                        if (ray_setup(cam, P->T, vsinv, __ldg(znear + (y >> 3) * zw + (x >> 3)),
-                                      __ldg(zfar + (y >> 3) * zw + (x >> 3)), __ldg(fnear + (y >> kFineShift) * fw + (x >> kFineShift)),
-                                      x, y, R))
-                            active = true;
-                        else
-                            vmap[(size_t)y * vpitch + x] = miss;
-                    }
-                }
-            }
-        }
-        if (__ballot_sync(0xffffffffu, active) == 0u) {
-            if (drained) break;
-            continue;
-        }
-        if (active && ray_step(rd, rstep, R)) {
-            vmap[(size_t)y * vpitch + x] = ray_finish(rd, rstep, vsinv, P->Tinv, R);
-            active = false;
-        }
+        unsigned t = 0u;
+        if (lane == 0) t = atomicAdd(queue, 1u);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= tiles) return;
+        const int x = (int)(t % (unsigned)tiles_x) * 8 + (lane & 7), y = (int)(t / (unsigned)tiles_x) * 4 + (lane >> 3);
+        march_pixel<FMT>(m, cam, P, znear, zfar, zw, vmap, vpitch, skipped, fnear, fw, g, x, y, -1);
     }
 }
 
@@ -476,51 +547,61 @@ static int march_resident_ctas(int fmt) {
 static void launch_march_persistent(const MapDev &m, int fmt, const Cam &cam, const PosePair *P,
                                     const RaycastBuffers &rb, float4 *vmap, int vmap_pitch_elems, const int *skip,
                                     cudaStream_t s) {
-    const unsigned total = (unsigned)(((cam.w + 7) / 8) * ((cam.h + 3) / 4) * 32);
-    const int grid = std::min(march_resident_ctas(fmt), (int)((total + 127) / 128));
+    const unsigned tiles = (unsigned)(((cam.w + 7) / 8) * ((cam.h + 3) / 4));
+    const int grid = std::min(march_resident_ctas(fmt), (int)((tiles + 3) / 4));
     switch (fmt) {
         case YAS_VOXEL_F32:
             march_persistent_kernel<YAS_VOXEL_F32><<<grid, 128, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, vmap,
-                                                                        vmap_pitch_elems, skip, rb.queue, total, rb.fnear, rb.fw);
+                                                                        vmap_pitch_elems, skip, rb.fnear, rb.fw, rb.grid, rb.queue, tiles);
             break;
         case YAS_VOXEL_F16:
             march_persistent_kernel<YAS_VOXEL_F16><<<grid, 128, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, vmap,
-                                                                        vmap_pitch_elems, skip, rb.queue, total, rb.fnear, rb.fw);
+                                                                        vmap_pitch_elems, skip, rb.fnear, rb.fw, rb.grid, rb.queue, tiles);
             break;
         case YAS_VOXEL_S16:
             march_persistent_kernel<YAS_VOXEL_S16><<<grid, 128, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, vmap,
-                                                                        vmap_pitch_elems, skip, rb.queue, total, rb.fnear, rb.fw);
+                                                                        vmap_pitch_elems, skip, rb.fnear, rb.fw, rb.grid, rb.queue, tiles);
             break;
         default:
             march_persistent_kernel<YAS_VOXEL_S24><<<grid, 128, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, vmap,
-                                                                        vmap_pitch_elems, skip, rb.queue, total, rb.fnear, rb.fw);
+                                                                        vmap_pitch_elems, skip, rb.fnear, rb.fw, rb.grid, rb.queue, tiles);
             break;
+    }
+}
+
+template <int WX, int WY, int RAYS>
+static void launch_march_rays(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, const RaycastBuffers &rb,
+                              float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s) {
+    constexpr int TX = (RAYS == 32 ? 8 : 4) * WX, TY = RAYS / (RAYS == 32 ? 8 : 4) * WY;
+    const dim3 grid((cam.w + TX - 1) / TX, (cam.h + TY - 1) / TY, 2);
+    const auto launch = [&](auto kernel) {
+        kernel<<<grid, 32 * WX * WY, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, vmap, vmap_pitch_elems, skip, rb.fnear,
+                                             rb.fw, rb.grid);
+    };
+    switch (fmt) {
+        case YAS_VOXEL_F32: launch(march_kernel<YAS_VOXEL_F32, WX, WY, RAYS>); break;
+        case YAS_VOXEL_F16: launch(march_kernel<YAS_VOXEL_F16, WX, WY, RAYS>); break;
+        case YAS_VOXEL_S16: launch(march_kernel<YAS_VOXEL_S16, WX, WY, RAYS>); break;
+        default: launch(march_kernel<YAS_VOXEL_S24, WX, WY, RAYS>); break;
     }
 }
 
 template <int WX, int WY>
 static void launch_march_tile(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, const RaycastBuffers &rb,
                               float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s) {
-    dim3 grid((cam.w + 8 * WX - 1) / (8 * WX), (cam.h + 4 * WY - 1) / (4 * WY));
-    const int threads = 32 * WX * WY;
-    switch (fmt) {
-        case YAS_VOXEL_F32:
-            march_kernel<YAS_VOXEL_F32, WX, WY><<<grid, threads, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, vmap,
-                                                                         vmap_pitch_elems, skip, rb.fnear, rb.fw);
-            break;
-        case YAS_VOXEL_F16:
-            march_kernel<YAS_VOXEL_F16, WX, WY><<<grid, threads, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, vmap,
-                                                                         vmap_pitch_elems, skip, rb.fnear, rb.fw);
-            break;
-        case YAS_VOXEL_S16:
-            march_kernel<YAS_VOXEL_S16, WX, WY><<<grid, threads, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, vmap,
-                                                                         vmap_pitch_elems, skip, rb.fnear, rb.fw);
-            break;
-        default:
-            march_kernel<YAS_VOXEL_S24, WX, WY><<<grid, threads, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, vmap,
-                                                                         vmap_pitch_elems, skip, rb.fnear, rb.fw);
-            break;
-    }
+    // Rays per warp.  A small image does not fill the GPU with warps of 32 rays,
+    // so a march lasts as long as its slowest warp, and that one ends sooner
+    // with fewer rays: 320x240, 8 mm: 56 us at 32 rays, 50 at 16 and 49 at 8;
+    // 160x120, 1 cm: 51 at 32 and 38 at 8.  In larger images instruction issue
+    // counts, and full warps take the fewest: 640x480, 5 mm: 79 us at 32, 96 at
+    // 16, 149 at 8.
+    const int px = cam.w * cam.h;
+    if (px <= 40000)
+        launch_march_rays<WX, WY, 8>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s);
+    else if (px <= 160000)
+        launch_march_rays<WX, WY, 16>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s);
+    else
+        launch_march_rays<WX, WY, 32>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s);
 }
 
 void launch_march(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, const RaycastBuffers &rb,

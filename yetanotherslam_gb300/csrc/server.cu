@@ -90,7 +90,8 @@ size_t session_bytes_estimate(const yas_session_config &c) {
     const size_t P0 = (size_t)c.width * c.height;
     const size_t pyramids = 88 * P;                       // two frame sets + gradients
     const size_t frame = P0 * (16 + 4 + 16 + 4 + 3 + 2 + 4); // residuals, staging, vmap, depth, inputs
-    return map + pyramids + frame + (8u << 20);            // + tracker rows, graphs, small buffers
+    const size_t grids = 2 * (size_t)kGridCells * 4;      // block grids of the frames' raycast and the raycaster
+    return map + pyramids + frame + grids + (8u << 20);   // + tracker rows, graphs, small buffers
 }
 
 }  // namespace

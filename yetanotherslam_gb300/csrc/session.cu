@@ -172,6 +172,8 @@ struct yas_session {
     // its raycaster between frames leave them alone): filled after each
     // frame's visibility pass, which is at the pose the next raycast uses
     RaycastBuffers zt = {};
+    // the map's edit count that zt's block grid covers
+    unsigned long long grid_edits = 0;
     yas_tracker *tr = nullptr;
     uint8_t *d_rgb = nullptr;
     uint16_t *d_depth = nullptr;
@@ -472,7 +474,10 @@ static int build_graph(yas_session *s, int parity) {
 // ---------------------------------------------------------------- interface for the request server
 namespace yas {
 
+static int refresh_grid(yas_session *s);
+
 int session_copy_input(yas_session *s, const uint8_t *rgb, const uint16_t *depth, int on_device) {
+    YAS_TRY(refresh_grid(s));
     const size_t n = (size_t)s->cfg.width * s->cfg.height;
     const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     YAS_TRY_CUDA(cudaMemcpyAsync(s->d_rgb, rgb, n * 3, kind, s->stream));
@@ -495,17 +500,32 @@ static void drop_graphs(yas_session *s) {
     s->post_exec = nullptr;
 }
 
-// Drops captured graphs that name map arrays which have since moved; a
-// hibernated map cannot run frames.
+// Makes the next raycast's block grid anew when calls on the map between
+// frames (an import, a fusion at another pose, a reset) may have changed its
+// blocks since.
+static int refresh_grid(yas_session *s) {
+    const unsigned long long edits = s->map->edits;
+    if (edits == s->grid_edits) return YAS_OK;
+    s->grid_edits = edits;
+    if (s->frames == 0) return YAS_OK;  // the initialising frame does not raycast
+    launch_block_grid(map_view(s->map), &s->fs->pp, s->zt, s->stream);
+    YAS_TRY_CUDA(cudaGetLastError());
+    return YAS_OK;
+}
+
+// Readies a session for a frame: drops captured graphs that name map arrays
+// which have since moved, and brings the next raycast up to date with the map;
+// a hibernated map cannot run frames.
 static int check_graphs(yas_session *s) {
     if (s->map->hibernated) return YAS_ERR_STATE;
     const void *now[5] = {s->map->slots, s->map->block_keys, s->map->voxels, s->map->visible, s->map->hdr};
     bool same = true;
     for (int i = 0; i < 5; ++i) same = same && now[i] == s->graph_arrays[i];
-    if (same) return YAS_OK;
-    drop_graphs(s);
-    for (int i = 0; i < 5; ++i) s->graph_arrays[i] = now[i];
-    return YAS_OK;
+    if (!same) {
+        drop_graphs(s);
+        for (int i = 0; i < 5; ++i) s->graph_arrays[i] = now[i];
+    }
+    return refresh_grid(s);
 }
 
 int session_launch_first(yas_session *s) {
@@ -618,22 +638,7 @@ YAS_API int yas_session_create(yas_session **out, const yas_session_config *cfg,
     s->cam = make_cam(cfg->K.fx, cfg->K.fy, cfg->K.cx, cfg->K.cy, cfg->width, cfg->height);
     int st = yas_map_create(&s->map, &cfg->map, &cfg->K, s->stream);
     if (st == YAS_OK) st = yas_raycaster_create(&s->rc, cfg->width, cfg->height, &cfg->K, s->stream);
-    if (st == YAS_OK) {
-        RaycastBuffers &z = s->zt;
-        z.w = cfg->width;
-        z.h = cfg->height;
-        z.zw = (cfg->width + 7) / 8;
-        z.zh = (cfg->height + 7) / 8;
-        z.fw = (cfg->width + (1 << kFineShift) - 1) >> kFineShift;
-        z.fh = (cfg->height + (1 << kFineShift) - 1) >> kFineShift;
-        const size_t nz = (size_t)z.zw * z.zh;
-        if (cudaMalloc(&z.znear, nz * 4) != cudaSuccess || cudaMalloc(&z.zfar, nz * 4) != cudaSuccess ||
-            cudaMalloc(&z.queue, sizeof(unsigned)) != cudaSuccess ||
-            cudaMalloc(&z.fnear, (size_t)z.fw * z.fh * 4) != cudaSuccess) {
-            cudaGetLastError();
-            st = YAS_ERR_OOM;
-        }
-    }
+    if (st == YAS_OK) st = raycast_buffers_alloc(s->zt, cfg->width, cfg->height);
     if (st == YAS_OK) {
         const double K[9] = {cfg->K.fx, 0, cfg->K.cx, 0, cfg->K.fy, cfg->K.cy, 0, 0, 1};
         st = yas_tracker_create(&s->tr, cfg->width, cfg->height, K, cfg->num_levels, cfg->iterations, cfg->mode,
@@ -678,10 +683,7 @@ YAS_API int yas_session_destroy(yas_session *s) {
     drop_graphs(s);
     if (s->tr) yas_tracker_destroy(s->tr);
     if (s->rc) yas_raycaster_destroy(s->rc);
-    cudaFree(s->zt.znear);
-    cudaFree(s->zt.zfar);
-    cudaFree(s->zt.queue);
-    cudaFree(s->zt.fnear);
+    raycast_buffers_free(s->zt);
     if (s->map) yas_map_destroy(s->map);
     cudaFree(s->d_rgb);
     cudaFree(s->d_depth);
@@ -794,6 +796,7 @@ YAS_API int yas_session_new_submap(yas_session *s, yas_map **out_previous) {
     // the next raycast's z-range tiles are the new (empty) map's
     frame_begin_kernel<<<1, 32, 0, s->stream>>>(s->fs, pose_identity(), nm->hdr);
     launch_zrange(map_view(nm), s->rc->cam, &s->fs->pp, s->zt, nullptr, s->stream);
+    s->grid_edits = nm->edits;
     YAS_TRY_CUDA(cudaGetLastError());
     YAS_TRY_CUDA(cudaMemcpyAsync(s->fs_host, s->fs, sizeof(FrameState), cudaMemcpyDeviceToHost, s->stream));
     YAS_TRY_CUDA(cudaStreamSynchronize(s->stream));

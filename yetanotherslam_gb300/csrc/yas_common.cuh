@@ -29,6 +29,10 @@ constexpr int kMaxProbes = 2048;   // bounded linear probing (no unbounded spin)
 constexpr int kSMs = 152;
 // Fine near-bound cells of the ray march: 2^kFineShift pixels square.
 constexpr int kFineShift = 2;
+// Block grid of a raycast: blocks per side, blocks.  160 blocks span the 3 m
+// view frustum in any orientation at 5 mm voxels and most of it at 4 mm.
+constexpr int kGridSide = 160;
+constexpr int kGridCells = kGridSide * kGridSide * kGridSide;
 constexpr int kCoordBits = 21;
 constexpr int kCoordMax = (1 << (kCoordBits - 1)) - 1;   // 1048575
 constexpr int kCoordMin = -(1 << (kCoordBits - 1));      // -1048576
@@ -116,8 +120,7 @@ struct __align__(16) MapHeader {
     unsigned n_visible;     // length of the visible list
     unsigned err_bits;      // sticky yas_status bits
     unsigned n_alloc_prev;  // n_alloc before the latest allocation pass
-    unsigned n_render;      // raycast: z-range tiles written
-    unsigned pad[3];
+    unsigned pad[4];
 };
 
 // ------------------------------------------------------------------ formats

@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <mutex>
 #include <string>
@@ -93,6 +94,11 @@ void launch_map_import(const MapDev &m, int fmt, const int *coords, const float 
 void launch_visible_coords(const MapDev &m, int *coords, unsigned count, cudaStream_t s);
 
 // ------------------------------------------------------------------ raycast.cu
+// The blocks around a raycast's view (raycast.cu).
+struct BlockGrid {
+    unsigned *cells;  // pool index of each block, tagged with the epoch
+    int *info;        // first block and epochs
+};
 struct RaycastBuffers {
     int w, h;          // image size
     int zw, zh;        // z-range map size: ceil(w/8), ceil(h/8)
@@ -101,9 +107,17 @@ struct RaycastBuffers {
     unsigned *queue;   // next pixel of the persistent march (reset with the z-range)
     int fw, fh;        // fine near-bound map size: ceil(w/4), ceil(h/4)
     float *fnear;      // fw*fh: nearest visible block whose projected box covers the 4x4 pixels
+    BlockGrid grid;
 };
+int raycast_buffers_alloc(RaycastBuffers &rb, int width, int height);
+void raycast_buffers_free(RaycastBuffers &rb);
+// Z-range tiles of the visible list and the block grid of the allocated blocks,
+// for a march at the same pose.
 void launch_zrange(const MapDev &m, const Cam &cam, const PosePair *P, RaycastBuffers &rb,
                    const int *skip, cudaStream_t s);
+// The block grid alone, for a map whose blocks changed between launch_zrange
+// and the march.
+void launch_block_grid(const MapDev &m, const PosePair *P, const RaycastBuffers &rb, cudaStream_t s);
 // `warps_x` 1, 2 (the default), 4: one thread per pixel, a 128-thread CTA's
 // four 8x4-pixel warp tiles side by side in x (8x16, 16x8, 32x4 pixels);
 // 0: persistent warps taking 8x4-pixel tiles from a queue.  The output is
@@ -150,6 +164,9 @@ struct yas_map {
     std::mutex pose_mutex;
     bool active = true;
     std::mutex active_mutex;
+    // counts the calls that may have changed the block set outside a session's
+    // frames: a session's next raycast looks blocks up in a grid made before
+    std::atomic<unsigned long long> edits{0};
     bool hibernated = false;
     std::vector<unsigned char> hib_slots, hib_keys, hib_voxels, hib_visible;
     yas::MapHeader hib_hdr;
