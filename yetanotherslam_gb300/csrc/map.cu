@@ -205,16 +205,39 @@ void launch_visible(const MapDev &m, const Cam &cam, const PosePair *P, const in
 
 // ---------------------------------------------------------------- integration
 // Pixel index floor(((a / z) + c) + 0.5) with the IEEE quotient a / z, as the
-// canonical FP32 order defines it.  The quotient is first formed as a * (1/z)
-// with the correctly rounded reciprocal (within 2 ulp of a / z); only when the
-// resulting coordinate lies within 8 ulp of an integer, where the two could
-// round to different pixels, is the exact division evaluated.
-__device__ __forceinline__ int project_exact(float a, float z, float rz, float c) {
-    const float t = cadd(cadd(cmul(a, rz), c), 0.5f);
-    const float ft = floorf(t);
-    const float tol = 8.0f * fmaxf(fabsf(t), fabsf(t - c)) * 1.1920929e-7f;
-    if (fabsf(t) < 8.0e6f && t - ft > tol && ft + 1.0f - t > tol) return (int)ft;
+// canonical FP32 order defines it: the exact form.
+__device__ __forceinline__ int project_exact(float a, float z, float c) {
     return f2i_floor(cadd(cadd(cdiv(a, z), c), 0.5f));
+}
+
+// Approximate FP32 reciprocal (relative error at most 2^-23).
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Largest distance of the coordinate s = a rcp_approx(z) + c from an integer at
+// which rint(s) is still the exact form's pixel, in an image `n` pixels wide.
+// The approximate quotient is within 2^-22 of a / z (reciprocal 2^-23, product
+// and IEEE quotient 2^-24 each) and the sums on either side round to within
+// 2^-24 of their results, so s + 0.5 differs from the exact form's last sum by
+// at most 2^-22 (2 |s| + |c| + 2); nearer than that to a pixel's edge, the
+// exact form is evaluated (about one voxel in 500 at 640x480).  Outside the
+// image the difference grows with |s| but stays far below its distance to the
+// image, up to 2^18 pixels; beyond (-1) every coordinate is evaluated exactly.
+__device__ __forceinline__ float project_margin(int n, float c) {
+    const float m = 2.0f * (float)n + fabsf(c) + 4.0f;
+    return m < 262144.0f ? 0.5f - m * 0x1p-22f : -1.0f;
+}
+
+// rint(s) of a pair by adding 1.5 * 2^23, and s's distance from it: no
+// conversion, which would take the quarter-rate pipe.  |s| < 2^22; a larger one
+// (or a NaN) comes back as a pixel outside every image or with a NaN distance.
+__device__ __forceinline__ int2 nearest_pixel2(float2 s, float2 &off) {
+    const float2 k = cadd2(s, pair(12582912.0f));
+    off = csub2(s, cadd2(k, pair(-12582912.0f)));
+    return make_int2(__float_as_int(k.x) - 0x4b400000, __float_as_int(k.y) - 0x4b400000);
 }
 
 // Each 128-thread group owns one block; thread t updates voxels 4t..4t+3
@@ -223,6 +246,12 @@ __device__ __forceinline__ int project_exact(float a, float z, float rz, float c
 // observation removed again (de-integration, for re-integration after a pose
 // correction): s <- (s w - d) / (w - 1), w <- w - 1; exact while the weight
 // stayed below the cap, as the reference's running average is then invertible.
+// Bound by instruction issue (the depth image and the blocks are in L2): a
+// thread projects its four voxels two at a time with packed FP32, starts their
+// depth reads, and then updates all four under one branch.  13 k visible blocks
+// at 640x480, 5 mm F16: 37.8 -> 25.6 us (80 % of the issue slots; before, a
+// correctly rounded reciprocal, conversions and a branch per voxel), 1280x720,
+// 4 mm F16: 59.8 -> 39.7, 320x240, 8 mm F32: 15.7 -> 12.6.
 template <int FMT, int SIGN>
 __global__ void __launch_bounds__(256) integrate_kernel(MapDev m, const float *__restrict__ depth,
                                                         int pitch, Cam cam, const PosePair *P,
@@ -236,6 +265,7 @@ __global__ void __launch_bounds__(256) integrate_kernel(MapDev m, const float *_
     const int t = threadIdx.x & 127;
     const int lz = t >> 4, ly = (t >> 1) & 7, lx0 = (t & 1) * 4;
     const float vs = m.voxel_size, inv_trunc = 1.0f / m.trunc, ntrunc = -m.trunc;
+    const float mar_u = project_margin(cam.w, cam.cx), mar_v = project_margin(cam.h, cam.cy);
     V *vox = static_cast<V *>(m.voxels);
     for (unsigned j = blockIdx.x * 2 + (threadIdx.x >> 7); j < nvis; j += gridDim.x * 2) {
         const int b = m.visible[j];
@@ -259,60 +289,97 @@ __global__ void __launch_bounds__(256) integrate_kernel(MapDev m, const float *_
         }
         const float wy = cmul((float)(by * 8 + ly), vs);
         const float wz = cmul((float)(bz * 8 + lz), vs);
-        bool dirty = false;
+        const float x0 = (float)(bx * 8 + lx0);
+        // the products of the rows with wy and wz are the same for all four
+        const float xy = cmul(Tinv.r[1], wy), xz = cmul(Tinv.r[2], wz), yy = cmul(Tinv.r[4], wy), yz = cmul(Tinv.r[5], wz);
+        const float zy = cmul(Tinv.r[7], wy), zz = cmul(Tinv.r[8], wz);
+        float au[4], av[4], zc[4], dist[4];
+        int u[4], w[4];
+        bool edge[4];
+#pragma unroll
+        for (int q = 0; q < 4; q += 2) {
+            // rigid_exact and the projection of a pair
+            const float2 wx = cmul2(cadd2(pair(x0), make_float2((float)q, (float)(q + 1))), pair(vs));  // x0 + q is exact
+            const float2 cx = cadd2(cadd2(cadd2(cmul_each(pair(Tinv.r[0]), wx), pair(xy)), pair(xz)), pair(Tinv.t[0]));
+            const float2 cy = cadd2(cadd2(cadd2(cmul_each(pair(Tinv.r[3]), wx), pair(yy)), pair(yz)), pair(Tinv.t[1]));
+            const float2 cz = cadd2(cadd2(cadd2(cmul_each(pair(Tinv.r[6]), wx), pair(zy)), pair(zz)), pair(Tinv.t[2]));
+            const float2 a = cmul2(pair(cam.fx), cx), b2 = cmul2(pair(cam.fy), cy);
+            const float2 rz = make_float2(rcp_approx(cz.x), rcp_approx(cz.y));
+            float2 off_u, off_v;
+            const int2 iu = nearest_pixel2(cadd2(cmul_each(a, rz), pair(cam.cx)), off_u);
+            const int2 iv = nearest_pixel2(cadd2(cmul_each(b2, rz), pair(cam.cy)), off_v);
+            edge[q] = !(fabsf(off_u.x) < mar_u && fabsf(off_v.x) < mar_v);
+            edge[q + 1] = !(fabsf(off_u.y) < mar_u && fabsf(off_v.y) < mar_v);
+            au[q] = a.x, au[q + 1] = a.y, av[q] = b2.x, av[q + 1] = b2.y;
+            zc[q] = cz.x, zc[q + 1] = cz.y;
+            u[q] = iu.x, u[q + 1] = iu.y, w[q] = iv.x, w[q + 1] = iv.y;
+        }
+        if (edge[0] || edge[1] || edge[2] || edge[3]) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (!edge[q]) continue;
+                u[q] = project_exact(au[q], zc[q], cam.cx);
+                w[q] = project_exact(av[q], zc[q], cam.cy);
+            }
+        }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const float wx = cmul((float)(bx * 8 + lx0 + q), vs);
-            float3 pc = rigid_exact(Tinv, wx, wy, wz);
-            const float rz = __frcp_rn(pc.z);
-            int u = project_exact(cmul(cam.fx, pc.x), pc.z, rz, cam.cx);
-            int vv = project_exact(cmul(cam.fy, pc.y), pc.z, rz, cam.cy);
-            if (u < 0 || vv < 0 || u > cam.w - 1 || vv > cam.h - 1) continue;
-            float dist = __ldg(depth + (size_t)vv * pitch + u);
-            if (isnan(dist) || dist > m.depth_max || dist < m.depth_min) continue;
-            float sdf = csub(dist, pc.z);
-            if (sdf < ntrunc) continue;
-            sdf = fminf(1.0f, sdf * inv_trunc);
-            int w = IO::wt(v[q]);
-            float ns;
-            if (SIGN > 0) {
-                if (w == 0) {
-                    ns = sdf;
-                    w = 1;
-                } else {
-                    ns = __fdividef(fmaf(IO::sdf(v[q]), (float)w, sdf), (float)(w + 1));
-                    w = min(m.max_weight, w + 1);
-                }
-            } else {
-                if (w == 0) continue;
-                if (w == 1) {
-                    ns = 0.0f;
-                    w = 0;
-                } else {
-                    ns = __fdividef(fmaf(IO::sdf(v[q]), (float)w, -sdf), (float)(w - 1));
-                    w = w - 1;
-                }
-            }
-            v[q] = IO::make(ns, w);
-            dirty = true;
+            dist[q] = __int_as_float(0x7fffffff);
+            if ((unsigned)u[q] < (unsigned)cam.w && (unsigned)w[q] < (unsigned)cam.h)
+                dist[q] = __ldg(depth + (size_t)w[q] * pitch + u[q]);
         }
-        if (dirty) {
-            if (sizeof(V) == 4) {
-                uint4 q;
-                q.x = *reinterpret_cast<unsigned *>(&v[0]);
-                q.y = *reinterpret_cast<unsigned *>(&v[1]);
-                q.z = *reinterpret_cast<unsigned *>(&v[2]);
-                q.w = *reinterpret_cast<unsigned *>(&v[3]);
-                *reinterpret_cast<uint4 *>(p) = q;
+        float d[4];
+        bool ok[4], any = false;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            d[q] = csub(dist[q], zc[q]);
+            ok[q] = dist[q] >= m.depth_min && dist[q] <= m.depth_max && !(d[q] < ntrunc);
+            if (SIGN < 0) ok[q] = ok[q] && IO::wt(v[q]) != 0;
+            any = any || ok[q];
+        }
+        if (!any) continue;
+        float ns[4];
+        int nw[4];
+        bool plain = true;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            // (the approximate quotient's error is two ulps)
+            const float sdf = fminf(1.0f, d[q] * inv_trunc), wf = IO::wtf(v[q]);
+            const int wt = IO::wt(v[q]);
+            const float up = SIGN > 0 ? fmaf(IO::sdf(v[q]), wf, sdf) * rcp_approx(wf + 1.0f)
+                                      : fmaf(IO::sdf(v[q]), wf, -sdf) * rcp_approx(wf - 1.0f);
+            if (SIGN > 0) {
+                ns[q] = wt == 0 ? sdf : up;
+                nw[q] = wt == 0 ? 1 : min(m.max_weight, wt + 1);
             } else {
-                float4 q0, q1;
-                *reinterpret_cast<V *>(&q0.x) = v[0];
-                *reinterpret_cast<V *>(&q0.z) = v[1];
-                *reinterpret_cast<V *>(&q1.x) = v[2];
-                *reinterpret_cast<V *>(&q1.z) = v[3];
-                reinterpret_cast<float4 *>(p)[0] = q0;
-                reinterpret_cast<float4 *>(p)[1] = q1;
+                ns[q] = wt == 1 ? 0.0f : up;
+                nw[q] = wt - 1;
             }
+            plain = plain && (!ok[q] || IO::plain(ns[q]));
+        }
+        if (plain) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = ok[q] ? IO::make_plain(ns[q], nw[q]) : v[q];
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (ok[q]) v[q] = IO::make(ns[q], nw[q]);
+        }
+        if (sizeof(V) == 4) {
+            uint4 q;
+            q.x = *reinterpret_cast<unsigned *>(&v[0]);
+            q.y = *reinterpret_cast<unsigned *>(&v[1]);
+            q.z = *reinterpret_cast<unsigned *>(&v[2]);
+            q.w = *reinterpret_cast<unsigned *>(&v[3]);
+            *reinterpret_cast<uint4 *>(p) = q;
+        } else {
+            float4 q0, q1;
+            *reinterpret_cast<V *>(&q0.x) = v[0];
+            *reinterpret_cast<V *>(&q0.z) = v[1];
+            *reinterpret_cast<V *>(&q1.x) = v[2];
+            *reinterpret_cast<V *>(&q1.z) = v[3];
+            reinterpret_cast<float4 *>(p)[0] = q0;
+            reinterpret_cast<float4 *>(p)[1] = q1;
         }
     }
 }

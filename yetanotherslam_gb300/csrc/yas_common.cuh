@@ -62,6 +62,36 @@ __device__ __forceinline__ float3 rigid_exact(const Rigid32 &T, float x, float y
     return o;
 }
 
+// Two values at a time: the packed FP32 instructions round each half as the
+// scalar ones do and take one issue slot for both.  The assembler contracts a
+// packed product with a packed sum in spite of their explicit rounding, so a
+// product that a sum follows is formed by two scalar ones (cmul_each).
+__device__ __forceinline__ float2 pair(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 cmul2(float2 a, float2 b) {
+    float2 d;
+    asm("{.reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mul.rn.f32x2 z, x, y; mov.b64 {%0, %1}, z;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 cmul_each(float2 a, float2 b) { return make_float2(cmul(a.x, b.x), cmul(a.y, b.y)); }
+__device__ __forceinline__ float2 cadd2(float2 a, float2 b) {
+    float2 d;
+    asm("{.reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 z, x, y; mov.b64 {%0, %1}, z;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 cfma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{.reg .b64 x, y, w, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 w, {%6, %7}; "
+        "fma.rn.f32x2 z, x, y, w; mov.b64 {%0, %1}, z;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 csub2(float2 a, float2 b) { return cfma2(b, pair(-1.0f), a); }
+
 // Fast form (FMA allowed) for continuous quantities compared with tolerance.
 __device__ __forceinline__ float3 rigid_fast(const Rigid32 &T, float x, float y, float z) {
     return make_float3(fmaf(T.r[0], x, fmaf(T.r[1], y, fmaf(T.r[2], z, T.t[0]))),
@@ -124,8 +154,13 @@ struct __align__(16) MapHeader {
 };
 
 // ------------------------------------------------------------------ formats
+// wt: the weight; wtf: the weight as a float (exact).  make: the word of (s, w);
+// make_plain: the same where plain(s), in fewer instructions.
 template <int FMT>
 struct VoxelIO;
+
+// A byte as a float without a conversion instruction (quarter rate).
+__device__ __forceinline__ float byte_float(unsigned b) { return __uint_as_float(0x4b000000u | b) - 8388608.0f; }
 
 template <>
 struct VoxelIO<YAS_VOXEL_F32> {
@@ -133,7 +168,10 @@ struct VoxelIO<YAS_VOXEL_F32> {
     static constexpr int kBytes = 8;
     __device__ __forceinline__ static float sdf(T v) { return v.x; }
     __device__ __forceinline__ static int wt(T v) { return (int)v.y; }
+    __device__ __forceinline__ static float wtf(T v) { return truncf(v.y); }
     __device__ __forceinline__ static T make(float s, int w) { return make_float2(s, (float)w); }
+    __device__ __forceinline__ static bool plain(float) { return true; }
+    __device__ __forceinline__ static T make_plain(float s, int w) { return make(s, w); }
 };
 
 // FP16 value + u8 weight, with the FP16 rounding residual in the word's spare
@@ -153,7 +191,23 @@ struct VoxelIO<YAS_VOXEL_F16> {
         return __int_as_float(__float_as_int(h) + q * 32);
     }
     __device__ __forceinline__ static int wt(T v) { return (int)(v >> 24); }
+    __device__ __forceinline__ static float wtf(T v) { return byte_float(v >> 24); }
+    // A plain s, 2^-14 <= |s| < 2 (a normal half): |s| rounded to 18 mantissa bits
+    // is U, in units of 32 of its FP32 bits; its 8 low bits are q, and U with q
+    // taken off is a half with its exponent bias moved.  Other values (zero,
+    // below a normal half, large) go the general way; the same words either way.
+    __device__ __forceinline__ static bool plain(float s) {
+        return (__float_as_uint(s) & 0x7fffffffu) - 0x38800000u < 0x40000000u - 0x38800000u;
+    }
+    __device__ __forceinline__ static T make_plain(float s, int w) {
+        const unsigned bits = __float_as_uint(s), U = ((bits & 0x7fffffffu) + 16u) >> 5;
+        return ((U + 128u - (0x1c000u << 8)) >> 8) | ((bits >> 16) & 0x8000u) | ((U & 0xffu) << 16) |
+               ((unsigned)min(w, 255) << 24);
+    }
     __device__ __forceinline__ static T make(float s, int w) {
+        return plain(s) ? make_plain(s, w) : make_general(s) | ((unsigned)min(w, 255) << 24);
+    }
+    __device__ __forceinline__ static T make_general(float s) {
         unsigned short hb = __half_as_ushort(__float2half_rn(s));
         int q = 0;
         if (hb & 0x7fffu) {  // h and s share the sign; d = |s| - |h| in FP32 bit units
@@ -168,7 +222,7 @@ struct VoxelIO<YAS_VOXEL_F16> {
             }
             q = max(-128, min(127, q));  // clamps only below the half's normal range
         }
-        return (unsigned)hb | (((unsigned)q & 0xffu) << 16) | ((unsigned)min(w, 255) << 24);
+        return (unsigned)hb | (((unsigned)q & 0xffu) << 16);
     }
 };
 
@@ -180,11 +234,14 @@ struct VoxelIO<YAS_VOXEL_S24> {
         return (float)((int)v >> 8) * (1.0f / 4194304.0f);
     }
     __device__ __forceinline__ static int wt(T v) { return (int)(v & 0xffu); }
+    __device__ __forceinline__ static float wtf(T v) { return byte_float(v & 0xffu); }
     __device__ __forceinline__ static T make(float s, int w) {
         int q = __float2int_rn(s * 4194304.0f);
         q = max(-8388608, min(8388607, q));
         return ((unsigned)q << 8) | ((unsigned)w & 0xffu);
     }
+    __device__ __forceinline__ static bool plain(float) { return true; }
+    __device__ __forceinline__ static T make_plain(float s, int w) { return make(s, w); }
 };
 
 // The reference's voxel (VoxelMap.h:26-30: short sdf, uchar wt, padded to 4
@@ -200,10 +257,13 @@ struct VoxelIO<YAS_VOXEL_S16> {
         return __fdiv_rn((float)(short)(v & 0xffffu), 32767.0f);
     }
     __device__ __forceinline__ static int wt(T v) { return (int)((v >> 16) & 0xffu); }
+    __device__ __forceinline__ static float wtf(T v) { return byte_float((v >> 16) & 0xffu); }
     __device__ __forceinline__ static T make(float s, int w) {
         const int q = max(-32767, min(32767, __float2int_rz(__fmul_rn(s, 32767.0f))));
         return ((unsigned)q & 0xffffu) | ((unsigned)min(w, 255) << 16);
     }
+    __device__ __forceinline__ static bool plain(float) { return true; }
+    __device__ __forceinline__ static T make_plain(float s, int w) { return make(s, w); }
 };
 
 // ------------------------------------------------------------------ map view
