@@ -38,46 +38,43 @@ __device__ __forceinline__ void ray_block(const Cam &c, const Rigid32 &T, float 
 // 3-D Bresenham walker over block coordinates with the reference's major-axis
 // choice and error terms (VoxelMap.cu:568-650).
 struct BlockLine {
-    int cur[3];
-    int inc[3];
-    int d2[3];   // 2*|d|
-    int major, a1, a2;
+    // components in the order major axis, a1, a2 (no indexing by axis, which
+    // would put them in local memory)
+    int cur[3], inc[3], d2[3];  // d2: 2 * |d|
+    int major;
     int err1, err2;
-    int count;   // number of blocks on the line (|d_major| + 1)
+    int count;  // number of blocks on the line (|d_major| + 1)
 
+    // (m, a1, a2) = (0, 1, 2), (1, 0, 2) or (2, 1, 0)
     __device__ __forceinline__ void init(const int s[3], const int e[3]) {
-        int ad[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            int d = e[i] - s[i];
-            cur[i] = s[i];
-            inc[i] = d < 0 ? -1 : 1;
-            ad[i] = d < 0 ? -d : d;
-            d2[i] = ad[i] << 1;
-        }
-        if (ad[0] >= ad[1] && ad[0] >= ad[2]) {
-            major = 0; a1 = 1; a2 = 2;
-        } else if (ad[1] >= ad[0] && ad[1] >= ad[2]) {
-            major = 1; a1 = 0; a2 = 2;
-        } else {
-            major = 2; a1 = 1; a2 = 0;
-        }
-        err1 = d2[a1] - 1;
-        err2 = d2[a2] - 1;
-        count = ad[major] + 1;
+        const int ax = abs(e[0] - s[0]), ay = abs(e[1] - s[1]), az = abs(e[2] - s[2]);
+        major = ax >= ay && ax >= az ? 0 : (ay >= ax && ay >= az ? 1 : 2);
+        const int sm = major == 0 ? s[0] : (major == 1 ? s[1] : s[2]), em = major == 0 ? e[0] : (major == 1 ? e[1] : e[2]);
+        const int s1 = major == 1 ? s[0] : s[1], e1 = major == 1 ? e[0] : e[1];
+        const int s2 = major == 2 ? s[0] : s[2], e2 = major == 2 ? e[0] : e[2];
+        cur[0] = sm, cur[1] = s1, cur[2] = s2;
+        inc[0] = em < sm ? -1 : 1, inc[1] = e1 < s1 ? -1 : 1, inc[2] = e2 < s2 ? -1 : 1;
+        d2[0] = abs(em - sm) << 1, d2[1] = abs(e1 - s1) << 1, d2[2] = abs(e2 - s2) << 1;
+        err1 = d2[1] - 1;
+        err2 = d2[2] - 1;
+        count = (d2[0] >> 1) + 1;
     }
     __device__ __forceinline__ void step() {
         if (err1 > 0) {
-            cur[a1] += inc[a1];
-            err1 -= d2[major];
+            cur[1] += inc[1];
+            err1 -= d2[0];
         }
         if (err2 > 0) {
-            cur[a2] += inc[a2];
-            err2 -= d2[major];
+            cur[2] += inc[2];
+            err2 -= d2[0];
         }
-        err1 += d2[a1];
-        err2 += d2[a2];
-        cur[major] += inc[major];
+        err1 += d2[1];
+        err2 += d2[2];
+        cur[0] += inc[0];
+    }
+    __device__ __forceinline__ int3 block() const {
+        return make_int3(major == 0 ? cur[0] : (major == 1 ? cur[1] : cur[2]), major == 1 ? cur[0] : cur[1],
+                         major == 2 ? cur[0] : cur[2]);
     }
 };
 
@@ -132,20 +129,34 @@ __global__ void __launch_bounds__(256) allocate_kernel(MapDev m, const float *__
             }
         }
     }
+    // Nearly all blocks of a frame are allocated already, so a step first looks
+    // them up (two at a time: their first probes are in flight together); only
+    // a warp with a lane whose block is missing goes through the insertion,
+    // which matches the lanes' keys and takes two counters' round trips.  A
+    // tracked frame at 640x480, 5 mm: 14 -> 9 us, 1280x720, 4 mm: 22 -> 16.
     const int nmax = __reduce_max_sync(0xffffffffu, n);
-    for (int s = 0; s < nmax; ++s) {
-        bool has = s < n;
-        unsigned long long key = kEmptyKey;
-        if (has) {
-            if (s > 0) line.step();
-            if (coord_in_range(line.cur[0], line.cur[1], line.cur[2])) {
-                key = pack_key(line.cur[0], line.cur[1], line.cur[2]);
+    for (int s = 0; s < nmax; s += 2) {
+        unsigned long long key[2] = {kEmptyKey, kEmptyKey}, found[2] = {kEmptyKey, kEmptyKey};
+        unsigned slot[2] = {0u, 0u};
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (s + i >= n) continue;
+            if (s + i > 0) line.step();
+            const int3 b = line.block();
+            if (coord_in_range(b.x, b.y, b.z)) {
+                key[i] = pack_key(b.x, b.y, b.z);
+                slot[i] = hash_key(key[i]) & m.slot_mask;
+                found[i] = __ldcg(&m.slots[slot[i]].key);
             } else {
                 raise_error(m, YAS_ERR_COORD_RANGE);
-                has = false;
             }
         }
-        warp_insert<VBYTES>(m, key, has);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            bool missing = found[i] != key[i];
+            if (missing && found[i] != kEmptyKey) missing = !probe_key(m, key[i], slot[i]);
+            if (__any_sync(0xffffffffu, missing)) warp_insert<VBYTES>(m, key[i], missing);
+        }
     }
 }
 

@@ -326,6 +326,19 @@ __device__ __forceinline__ int claim_slot(const MapDev &m, unsigned long long ke
     return -1;
 }
 
+// True if `key` is in the table, probing from slot s + 1 on (the caller has
+// seen that slot s holds another key).
+__device__ __forceinline__ bool probe_key(const MapDev &m, unsigned long long key, unsigned s) {
+#pragma unroll 1
+    for (int i = 1; i < kMaxProbes; ++i) {
+        s = (s + 1) & m.slot_mask;
+        const unsigned long long k = __ldcg(&m.slots[s].key);
+        if (k == key) return true;
+        if (k == kEmptyKey) return false;
+    }
+    return false;
+}
+
 __device__ __forceinline__ void raise_error(const MapDev &m, int code) {
     atomicOr(&m.hdr->err_bits, err_bit(code));
 }
