@@ -114,6 +114,12 @@ __device__ __forceinline__ int clamp_ceil(float v) {
     return (int)ceilf(v);
 }
 
+// The tiles of every visible block: eight lanes a block, one corner each, which
+// then share the block's cells (4x2 at a time).  Bound by its chain of
+// latencies and atomics; one thread a block did 8 projections and some 40
+// atomics one after the other, and counted its tiles on one shared counter
+// (with the reset, 13 k blocks at 640x480, 5 mm: 15.5 -> 12.5 us, with the
+// block grid's fill in it now).
 __global__ void __launch_bounds__(128) zrange_fill_kernel(MapDev m, Cam cam, const PosePair *P,
                                                           float *znear, float *zfar, int zw, int zh,
                                                           const int *skip, float *fnear, int fw, int fh,
@@ -123,59 +129,53 @@ __global__ void __launch_bounds__(128) zrange_fill_kernel(MapDev m, Cam cam, con
     const unsigned nvis = *(volatile unsigned *)&m.hdr->n_visible;
     const Rigid32 Tinv = P->Tinv;
     const float scale = m.voxel_size * 8.0f;
-    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < nvis; j += gridDim.x * blockDim.x) {
+    const unsigned lane = lane_id(), c = lane & 7u, shift = lane & ~7u;
+    const int lx = (int)(c & 3u), ly = (int)(c >> 2);
+    for (unsigned base = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / 8u; base < nvis;
+         base += gridDim.x * blockDim.x / 8u) {
+        const unsigned j = base + lane / 8u;
+        const bool have = j < nvis;
         int bx, by, bz;
-        unpack_key(m.block_keys[m.visible[j]], bx, by, bz);
-        int ulx = zw, uly = zh, lrx = -1, lry = -1;
-        float zmin = m.depth_max, zmax = m.depth_min;
-        float pu0 = 1e30f, pu1 = -1e30f, pv0 = 1e30f, pv1 = -1e30f;
-        bool behind = false;
+        unpack_key(m.block_keys[m.visible[have ? j : base]], bx, by, bz);
+        const float3 p = rigid_exact(Tinv, (float)(bx + (int)(c & 1u)) * scale, (float)(by + (int)((c >> 1) & 1u)) * scale,
+                                     (float)(bz + (int)(c >> 2)) * scale);
+        const float pu = cam.fx * p.x / p.z + cam.cx, pv = cam.fy * p.y / p.z + cam.cy;
+        const bool behind = ((__ballot_sync(0xffffffffu, !(p.z > 1e-3f)) >> shift) & 0xffu) != 0u;
+        // a NaN coordinate counts as far to the left and up, as clamp_floor has it
+        const bool nan_u = ((__ballot_sync(0xffffffffu, isnan(pu)) >> shift) & 0xffu) != 0u;
+        const bool nan_v = ((__ballot_sync(0xffffffffu, isnan(pv)) >> shift) & 0xffu) != 0u;
+        float pu0 = fminf(pu, 1e30f), pu1 = fmaxf(pu, -1e30f), pv0 = fminf(pv, 1e30f), pv1 = fmaxf(pv, -1e30f);
+        float zmin = fminf(m.depth_max, p.z), zmax = fmaxf(m.depth_min, p.z);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            float3 p = rigid_exact(Tinv, (float)(bx + (c & 1)) * scale, (float)(by + ((c >> 1) & 1)) * scale,
-                                   (float)(bz + ((c >> 2) & 1)) * scale);
-            const float pu = cam.fx * p.x / p.z + cam.cx, pv = cam.fy * p.y / p.z + cam.cy;
-            float u = pu / 8.0f;
-            float v = pv / 8.0f;
-            ulx = min(ulx, clamp_floor(u));
-            uly = min(uly, clamp_floor(v));
-            lrx = max(lrx, clamp_ceil(u));
-            lry = max(lry, clamp_ceil(v));
-            zmin = fminf(zmin, p.z);
-            zmax = fmaxf(zmax, p.z);
-            behind = behind || !(p.z > 1e-3f);
-            pu0 = fminf(pu0, pu);
-            pu1 = fmaxf(pu1, pu);
-            pv0 = fminf(pv0, pv);
-            pv1 = fmaxf(pv1, pv);
+        for (int o = 1; o < 8; o <<= 1) {
+            pu0 = fminf(pu0, __shfl_xor_sync(0xffffffffu, pu0, o));
+            pu1 = fmaxf(pu1, __shfl_xor_sync(0xffffffffu, pu1, o));
+            pv0 = fminf(pv0, __shfl_xor_sync(0xffffffffu, pv0, o));
+            pv1 = fmaxf(pv1, __shfl_xor_sync(0xffffffffu, pv1, o));
+            zmin = fminf(zmin, __shfl_xor_sync(0xffffffffu, zmin, o));
+            zmax = fmaxf(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
         }
+        if (!have || !(zmax >= m.depth_min)) continue;
         // Fine near bound (not a reference quantity; the march uses it only to
         // jump over samples that lie before every visible block along the ray):
         // the block's projected box widened by a pixel, or the whole image when a
         // corner is not in front of the camera.
-        if (zmax >= m.depth_min) {
-            int fx0 = 0, fy0 = 0, fx1 = fw - 1, fy1 = fh - 1;
-            if (!behind) {
-                constexpr float kInvCell = 1.0f / (float)(1 << kFineShift);
-                fx0 = max(fx0, clamp_floor((pu0 - 1.0f) * kInvCell));
-                fy0 = max(fy0, clamp_floor((pv0 - 1.0f) * kInvCell));
-                fx1 = min(fx1, clamp_floor((pu1 + 1.0f) * kInvCell));
-                fy1 = min(fy1, clamp_floor((pv1 + 1.0f) * kInvCell));
-            }
-            const int fz = __float_as_int(fmaxf(fminf(zmin, m.depth_max), 0.0f));
-            for (int y = fy0; y <= fy1; ++y)
-                for (int x = fx0; x <= fx1; ++x) atomicMin(reinterpret_cast<int *>(fnear) + y * fw + x, fz);
+        int fx0 = 0, fy0 = 0, fx1 = fw - 1, fy1 = fh - 1;
+        if (!behind) {
+            constexpr float kInvCell = 1.0f / (float)(1 << kFineShift);
+            fx0 = max(fx0, clamp_floor((pu0 - 1.0f) * kInvCell));
+            fy0 = max(fy0, clamp_floor((pv0 - 1.0f) * kInvCell));
+            fx1 = min(fx1, clamp_floor((pu1 + 1.0f) * kInvCell));
+            fy1 = min(fy1, clamp_floor((pv1 + 1.0f) * kInvCell));
         }
-        ulx = max(ulx, 0);
-        uly = max(uly, 0);
-        lrx = min(lrx, zw - 1);
-        lry = min(lry, zh - 1);
-        if (ulx > lrx || uly > lry) continue;
-        if (zmin < m.depth_min) zmin = m.depth_min;
-        if (zmax < m.depth_min) continue;
-        const int inear = __float_as_int(zmin), ifar = __float_as_int(zmax);
-        for (int y = uly; y <= lry; ++y)
-            for (int x = ulx; x <= lrx; ++x) {
+        const int fz = __float_as_int(fmaxf(fminf(zmin, m.depth_max), 0.0f));
+        for (int y = fy0 + ly; y <= fy1; y += 2)
+            for (int x = fx0 + lx; x <= fx1; x += 4) atomicMin(reinterpret_cast<int *>(fnear) + y * fw + x, fz);
+        const int ulx = max(nan_u ? 0 : clamp_floor(pu0 / 8.0f), 0), uly = max(nan_v ? 0 : clamp_floor(pv0 / 8.0f), 0);
+        const int lrx = min(clamp_ceil(pu1 / 8.0f), zw - 1), lry = min(clamp_ceil(pv1 / 8.0f), zh - 1);
+        const int inear = __float_as_int(fmaxf(zmin, m.depth_min)), ifar = __float_as_int(zmax);
+        for (int y = uly + ly; y <= lry; y += 2)
+            for (int x = ulx + lx; x <= lrx; x += 4) {
                 atomicMin(reinterpret_cast<int *>(znear) + y * zw + x, inear);
                 atomicMax(reinterpret_cast<int *>(zfar) + y * zw + x, ifar);
             }
@@ -221,7 +221,7 @@ void launch_zrange(const MapDev &m, const Cam &cam, const PosePair *P, RaycastBu
     const int n = rb.zw * rb.zh, nf = rb.fw * rb.fh;
     zrange_reset_kernel<<<(std::max(n, nf) + 255) / 256, 256, 0, s>>>(m, P, rb.znear, rb.zfar, n, rb.queue, rb.fnear,
                                                                       nf, rb.grid);
-    zrange_fill_kernel<<<kSMs * 2, 128, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, rb.zh, skip, rb.fnear, rb.fw,
+    zrange_fill_kernel<<<kSMs * 8, 128, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, rb.zh, skip, rb.fnear, rb.fw,
                                                rb.fh, rb.grid);
 }
 
