@@ -40,7 +40,8 @@ struct CachedStep {
 };
 
 struct GNGroup {
-    int item0, nitems, cta0, nctas, pix;
+    int item0, nitems, cta0, nctas;
+    GNBatchShape shape;
 };
 
 constexpr size_t kMaxCached = 8;
@@ -150,7 +151,7 @@ static int plan_gn(yas_batch *b, const std::vector<uint8_t> &key, std::vector<GN
         if (key[i] >= kTrack0) tracked.push_back(session_tracker(b->s[i]));
     auto close_group = [&](GNGroup &g) {
         if (!g.nitems) return;
-        g.pix = gn_batch_pix(items.data() + g.item0, g.nitems);
+        g.shape = gn_batch_shape(items.data() + g.item0, g.nitems);
         groups.push_back(g);
     };
     auto add = [&](GNGroup &g, yas_tracker *tr, int n) {
@@ -163,13 +164,13 @@ static int plan_gn(yas_batch *b, const std::vector<uint8_t> &key, std::vector<GN
     };
     const int ppc = b->tuning.gn_pixels_per_cta;
     if (ppc > 0) {
-        GNGroup g = {0, 0, 0, 0, 0};
+        GNGroup g = {0, 0, 0, 0, {}};
         for (yas_tracker *tr : tracked) {
             const int n = gn_batch_ctas(tr, ppc);
             if (n > capacity) return YAS_ERR_CAPACITY;
             if (g.nctas + n > capacity) {
                 close_group(g);
-                g = {(int)items.size(), 0, (int)cta_item.size(), 0, 0};
+                g = {(int)items.size(), 0, (int)cta_item.size(), 0, {}};
             }
             add(g, tr, n);
         }
@@ -207,7 +208,7 @@ static int plan_gn(yas_batch *b, const std::vector<uint8_t> &key, std::vector<GN
             ++n[best];
             ++sum;
         }
-        GNGroup g = {(int)items.size(), 0, (int)cta_item.size(), 0, 0};
+        GNGroup g = {(int)items.size(), 0, (int)cta_item.size(), 0, {}};
         for (size_t k = 0; k < m; ++k) add(g, tracked[g0 + k], n[k]);
         close_group(g);
     }
@@ -281,7 +282,7 @@ static int capture_step(yas_batch *b, const std::vector<uint8_t> &key, CachedSte
                 }
                 if (err == cudaSuccess)
                     err = launch_gn_batch(out.d_items + k, out.d_map, items[(size_t)k].nctas, st,
-                                          gn_batch_pix(&items[(size_t)k], 1));
+                                          gn_batch_shape(&items[(size_t)k], 1));
                 if (err == cudaSuccess) session_enqueue_post(s);
             }
         }
@@ -292,7 +293,7 @@ static int capture_step(yas_batch *b, const std::vector<uint8_t> &key, CachedSte
             if (key[i] >= kTrack0) err = cudaStreamWaitEvent(b->stream, b->ev_pre[i], 0);
         for (const GNGroup &g : groups) {
             if (err != cudaSuccess) break;
-            err = launch_gn_batch(out.d_items + g.item0, out.d_map + g.cta0, g.nctas, b->stream, g.pix);
+            err = launch_gn_batch(out.d_items + g.item0, out.d_map + g.cta0, g.nctas, b->stream, g.shape);
         }
         if (err == cudaSuccess && !groups.empty()) err = cudaEventRecord(b->ev_gn, b->stream);
         for (size_t i = 0; i < b->s.size() && err == cudaSuccess; ++i) {

@@ -1243,7 +1243,7 @@ YAS_API int yas_tracker_check_wait_limit(yas_tracker *tr, int *out_status) {
     if (e == cudaSuccess) e = cudaMemsetAsync(d_map, 0, 2 * sizeof(unsigned short), tr->stream);
     if (e == cudaSuccess) {
         launch_gn_init(tr, pose_identity(), tr->stream);
-        e = launch_gn_batch(d_item, d_map, 1, tr->stream, gn_batch_pix(&it, 1));
+        e = launch_gn_batch(d_item, d_map, 1, tr->stream, gn_batch_shape(&it, 1));
     }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(tr->state_host, tr->state, sizeof(GNState), cudaMemcpyDeviceToHost, tr->stream);

@@ -207,10 +207,28 @@ __device__ __forceinline__ float sel3f(int i, float x, float y, float z) { retur
 constexpr unsigned kAbsMaskF = 0x7fffffffu;
 constexpr unsigned kInfBitsF = 0x7f800000u;
 
+// The three series of the SE(3) exponential in FP64.
+__device__ __forceinline__ void exp_coefficients(DF th2, DF &cA, DF &cB, DF &cC) {
+    const double t2 = df_to_double(th2);
+    const double th = sqrt(t2);
+    double sn, cs;
+    sincos(th, &sn, &cs);
+    cA = df_from_double(sn / th);
+    cB = df_from_double((1.0 - cs) / t2);
+    cC = df_from_double((th - sn) / (t2 * th));
+}
+
+// What the solve rarely needs, out of line: a schedule kernel runs through its
+// whole code in every iteration, and its size counts.
+__device__ __noinline__ void exp_coefficients_call(DF th2, DF &cA, DF &cB, DF &cC) { exp_coefficients(th2, cA, cB, cC); }
+__device__ __noinline__ DF df_div_call(DF a, DF x) { return df_div(a, x); }
+
 // The solve (warp 0; every lane must call it).  Reads g_solve's totals and
 // estimate state, writes the new state and the outputs back to g_solve.
-// Inlined into kernels with registers to spare (gn_solve_inline), called
-// (gn_solve) from the 64-register ones, where inlining adds spills.
+// Inlined into kernels with registers to spare (gn_solve_inline, kApart: its
+// rare parts out of line), called (gn_solve) from the 64-register ones, where
+// inlining, or calls from it, add spills.
+template <bool kApart>
 __device__ __forceinline__ void gn_solve_inline(int mode, int no_update, int first_of_level, int level) {
     SolveShared &S = g_solve;
     constexpr unsigned kAll = 0xffffffffu;
@@ -311,7 +329,7 @@ __device__ __forceinline__ void gn_solve_inline(int mode, int no_update, int fir
         }
     }
     if (broke) {  // forward substitution with the unfactored lower triangle
-#pragma unroll
+#pragma unroll 1
         for (int j = 0; j < 5; ++j) {
             const DF yj = df_shfl(a, 21 + j);
             const bool u = isb && ei > j;
@@ -325,7 +343,7 @@ __device__ __forceinline__ void gn_solve_inline(int mode, int no_update, int fir
        // final once its step has run), a division when nothing was factorised
         const DF dd = df_shfl(a, isb ? tri_lane(ei, ei) : lane);
         const unsigned db = __float_as_uint(dd.h) & kAbsMaskF;
-        if (isb) a = (db != 0u && db < kInfBitsF) ? (broke ? df_div(a, dd) : df_mul(a, rk)) : df(0.0f);
+        if (isb) a = (db != 0u && db < kInfBitsF) ? (broke ? (kApart ? df_div_call(a, dd) : df_div(a, dd)) : df_mul(a, rk)) : df(0.0f);
     }
     // ---- L^T z = y: b_i -= L(j, i) z_j for j > i
 #pragma unroll
@@ -387,14 +405,11 @@ __device__ __forceinline__ void gn_solve_inline(int mode, int no_update, int fir
         cB = df_shfl(pc, 1);
         cC = df_shfl(pc, 2);
     } else {
-        // rotations above 0.1 rad per iteration: FP64 (rare)
-        const double t2 = df_to_double(th2);
-        const double th = sqrt(t2);
-        double sn, cs;
-        sincos(th, &sn, &cs);
-        cA = df_from_double(sn / th);
-        cB = df_from_double((1.0 - cs) / t2);
-        cC = df_from_double((th - sn) / (t2 * th));
+        // rotations above 0.1 rad per iteration (rare)
+        if constexpr (kApart)
+            exp_coefficients_call(th2, cA, cB, cC);
+        else
+            exp_coefficients(th2, cA, cB, cC);
     }
     const int i = lane < 12 ? lane >> 2 : 0, q = lane & 3;
     const bool tl = q == 3;
@@ -443,7 +458,7 @@ __device__ __forceinline__ void gn_solve_inline(int mode, int no_update, int fir
 }
 
 __device__ __noinline__ void gn_solve(int mode, int no_update, int first_of_level, int level) {
-    gn_solve_inline(mode, no_update, first_of_level, level);
+    gn_solve_inline<false>(mode, no_update, first_of_level, level);
 }
 
 // Threads 0..31 load the estimate state of `st` into g_solve (the caller sets

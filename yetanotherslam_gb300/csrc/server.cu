@@ -72,7 +72,8 @@ struct ServedSession {
     GNBatchItem *d_own = nullptr;  // gn_per_session: the session's descriptor per frame parity
     GNBatchItem *h_own = nullptr;  // pinned source of d_own, written once per parity
     bool own_ready[2] = {false, false};
-    int own_ctas = 0, own_pix = 0;
+    int own_ctas = 0;
+    GNBatchShape own_shape = {};
     cudaEvent_t ev_gn = nullptr;  // after the session's own GN launch
     bool gn_running = false;      // its share counts against the co-resident CTAs
     long long submitted = 0, completed = 0;
@@ -213,10 +214,10 @@ int launch_own_gn(yas_server *srv, ServedSession *ss) {
         gn_batch_item_ctas(tr, 0, own_share(srv, ss), &it);
         YAS_TRY_CUDA(cudaMemcpyAsync(ss->d_own + p, &it, sizeof(it), cudaMemcpyHostToDevice, st));
         ss->own_ctas = it.nctas;
-        ss->own_pix = gn_batch_pix(&it, 1);
+        ss->own_shape = gn_batch_shape(&it, 1);
         ss->own_ready[p] = true;
     }
-    YAS_TRY_CUDA(launch_gn_batch(ss->d_own + p, srv->d_zero_map, ss->own_ctas, st, ss->own_pix));
+    YAS_TRY_CUDA(launch_gn_batch(ss->d_own + p, srv->d_zero_map, ss->own_ctas, st, ss->own_shape));
     YAS_TRY_CUDA(cudaEventRecord(ss->ev_gn, st));
     ss->gn_running = true;
     srv->own_ctas_running += ss->own_ctas;
@@ -267,7 +268,7 @@ int dispatch_gn(yas_server *srv, const std::vector<ServedSession *> &batch) {
     YAS_TRY_CUDA(cudaMemcpyAsync(srv->d_map[k], srv->h_map[k], (size_t)cta0 * sizeof(unsigned short),
                                  cudaMemcpyHostToDevice, srv->gn_stream));
     YAS_TRY_CUDA(launch_gn_batch(srv->d_items[k], srv->d_map[k], cta0, srv->gn_stream,
-                                 gn_batch_pix(srv->h_items[k], (int)batch.size())));
+                                 gn_batch_shape(srv->h_items[k], (int)batch.size())));
     YAS_TRY_CUDA(cudaEventRecord(srv->gn_done[k], srv->gn_stream));
     for (ServedSession *ss : batch) {
         cudaStream_t st = session_stream(ss->s);

@@ -256,6 +256,16 @@ __device__ __forceinline__ void make_rkinv(const float *T, const LevelCam &c, fl
     }
 }
 
+// Entry e of it alone, the same operations.
+__device__ __forceinline__ void rkinv_entry(const float *T, const LevelCam &c, float *RK, int e) {
+    const int i = e / 3, j = e - 3 * i;
+    const float a = T[i * 4], b = T[i * 4 + 1];
+    const float cxi = __fmul_rn(c.cx, c.invfx), cyi = __fmul_rn(c.cy, c.invfy);
+    RK[e] = j == 0   ? __fmul_rn(a, c.invfx)
+            : j == 1 ? __fmul_rn(b, c.invfy)
+                     : __fsub_rn(__fsub_rn(T[i * 4 + 2], __fmul_rn(a, cxi)), __fmul_rn(b, cyi));
+}
+
 // ---------------------------------------------------------------- pixel math
 // TransformReferencePoint (ImageProc.cu:42-78): (RKinv (x,y,1)) z + t, fixed order.
 __device__ __forceinline__ float3 warp_ref_point(const float *RK, const float *T, int x, int y, float z) {
@@ -332,7 +342,7 @@ __device__ __forceinline__ bool icp_match(const float *T, const LevelCam &c, con
 // The ICP row [n, v x n | r] of a matched pair, accumulated into the 28
 // products (the r^2 term as the sum of rounded squares, as the oracle sums
 // it) and the count.
-__device__ __forceinline__ void icp_accumulate(const float3 &vl, const float3 &nl, float r, float acc[32]) {
+__device__ __forceinline__ void icp_accumulate(const float3 &vl, const float3 &nl, float r, float *acc) {
     float row[6];
     row[0] = nl.x;
     row[1] = nl.y;
@@ -359,6 +369,11 @@ __device__ __forceinline__ float bilinear(const float *__restrict__ m, int w, fl
            (__ldg(r1) * (1.0f - cx) + __ldg(r1 + 1) * cx) * cy;
 }
 
+// The same from the four neighbours and the fractions.
+__device__ __forceinline__ float lerp2(float a, float b, float c, float d, float cx, float cy) {
+    return (a * (1.0f - cx) + b * cx) * (1.0f - cy) + (c * (1.0f - cx) + d * cx) * cy;
+}
+
 // Huber threshold 4.685 * stddev of the photometric residuals, in FP32 as the
 // reference (RGBDTracking.cu:259-278), from the double-float totals
 // n = tot[29], sum r = tot[30], sum r^2 = tot[31]: mean = sum r / n, then
@@ -370,7 +385,11 @@ __device__ __forceinline__ float huber_threshold_df(DF nn, DF s, DF s2) {
     const DF md = df(mean);
     const DF ss = df_fma(df_mul(nn, md), md, df_fma(df(-2.0f * mean), s, s2));
     const float var = sqrtf(ss.h / (nn.h - 1.0f));
-    return (float)(4.685 * (double)var);
+    // 4.685 var from its product with 4.685 to 48 bits, rounded once (an FP64
+    // product costs three serial FP64 instructions of some 65 cycles each)
+    constexpr float ch = 4.685f, cl = (float)(4.685 - (double)ch);
+    const float p = __fmul_rn(ch, var);
+    return __fadd_rn(p, __fmaf_rn(cl, var, __fmaf_rn(ch, var, -p)));
 }
 __device__ __forceinline__ float huber_threshold(const double *tot) {
     return huber_threshold_df(df_from_double(tot[29]), df_from_double(tot[30]), df_from_double(tot[31]));
@@ -558,7 +577,7 @@ constexpr unsigned long long kWaitLimitNs = 1000000000ull;  // 1 s
 struct FusedArgs {
     FusedLevel lv[kMaxLevels];
     int L, mode;
-    float angle_th, dist_th;
+    IcpGates gates;
     unsigned long long *rows;  // [2 parities][2 passes][kFusedMaxCtas][32] tagged words
     float4 *res4;              // per-pixel residuals of the PIX == 0 schedule (level-0 sized)
     GNState *st;
@@ -594,8 +613,9 @@ __device__ __forceinline__ bool tag_is(unsigned long long w, unsigned tag) { ret
 
 // One step of a bounded poll: false once the launch was aborted or this
 // thread's wait (started at t0) exceeded kWaitLimitNs, which it then reports.
+// The first polls follow one another at once (most rows come with the second).
 __device__ __forceinline__ bool poll_continue(GNState *st, unsigned spin, unsigned long long &t0) {
-    __nanosleep(spin < 32 ? 32 : 256);
+    if (spin >= 4) __nanosleep(spin < 32 ? 32 : 256);
     if ((spin & 15u) != 15u) return true;
     if (ld_relaxed_u32(&st->abort_word) != 0u) return false;
     const unsigned long long now = global_ns();
@@ -609,51 +629,89 @@ __device__ __forceinline__ bool poll_continue(GNState *st, unsigned spin, unsign
     return true;
 }
 
-// Pass A for one pixel whose reference depth (1 / inverse depth, 0 where
-// that is invalid: the same division gn_pass_a makes) and model vertex are
-// already loaded: the photometric residual (kept in registers for pass B)
-// and the ICP products, accumulated as gn_pass_a does.
-__device__ __forceinline__ void fused_pixel_a_pre(const FusedLevel &lv, const float *sT, const float *sRK, int k,
-                                                  bool do_rgb, bool do_icp, float angle_th, float dist_th,
-                                                  float z, float4 vm, float acc[32], float4 &res, float3 &p) {
-    const LevelCam &c = lv.c;
-    const int y = k / c.w, x = k - y * c.w;
-    res = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-    p = make_float3(0.0f, 0.0f, 1.0f);
-    if (do_rgb) {
-        if (z > 0.0f) {
-            p = warp_ref_point(sRK, sT, x, y, z);
-            float u, v;
-            if (rgb_project(c, p, u, v)) {
-                const float r = bilinear(lv.cur_int, c.w, u, v) - __ldg(lv.ref_int + k);
-                const float gx = bilinear(lv.cur_gx, c.w, u, v);
-                const float gy = bilinear(lv.cur_gy, c.w, u, v);
-                const bool ok = (gx * gx + gy * gy) > 0.0f && isfinite(r);
-                res = make_float4(r, gx, gy, ok ? 1.0f : -1.0f);
-                if (ok) {
-                    acc[29] += 1.0f;
-                    acc[30] += r;
-                    acc[31] += r * r;
-                }
-            }
-        }
-    }
-    if (do_icp) {
-        float3 vl, nl;
-        float4 vc;
-        float r;
-        if (icp_match_vm(sT, c, vm, lv.ref_nmap, lv.cur_vmap, lv.cur_nmap, k, angle_th, dist_th, vl, nl, vc, r))
-            icp_accumulate(vl, nl, r, acc);
+// Row and column of pixel k of a level: the high product with ceil(2^32 / w)
+// exceeds k / w by less than a half (k < 2^31), so it is y or y + 1.
+__device__ __forceinline__ void pixel_of(const FusedLevel &lv, int k, int &x, int &y) {
+    y = (int)__umulhi((unsigned)k, lv.wdiv);
+    x = k - y * lv.c.w;
+    if (x < 0) {
+        x += lv.c.w;
+        --y;
     }
 }
 
-// Pass A for one pixel: the photometric residual (kept in registers for pass
-// B) and the ICP products, accumulated as gn_pass_a does.
-__device__ __forceinline__ void fused_pixel_a(const FusedLevel &lv, const float *sT, const float *sRK, int k,
-                                              bool do_rgb, bool do_icp, float angle_th, float dist_th,
-                                              float acc[32], float4 &res, float3 &p) {
-    fused_pixel_a_pre(lv, sT, sRK, k, do_rgb, do_icp, angle_th, dist_th, do_rgb ? __ldg(lv.ref_z + k) : 0.0f,
-                      do_icp ? __ldg(lv.ref_vmap + k) : make_float4(0.0f, 0.0f, 0.0f, -1.0f), acc, res, p);
+// Photometric half of pass A for one pixel (gn_pass_a's residual and moments)
+// whose reference depth (1 / inverse depth, 0 where that is invalid) is loaded.
+// Pixels that project outside read image pixel 0 and are dropped afterwards, so
+// the gathers of a thread's pixels do not wait for one another's branches.
+__device__ __forceinline__ void fused_pixel_rgb(const FusedLevel &lv, const float *sT, const float *sRK, int k, float z,
+                                                float sums[3], float4 &res, float3 &p) {
+    const LevelCam &c = lv.c;
+    int x, y;
+    pixel_of(lv, k, x, y);
+    p = warp_ref_point(sRK, sT, x, y, z);
+    float u, v;
+    const bool inside = rgb_project(c, p, u, v) && z > 0.0f;
+    const float fu = inside ? floorf(u) : 0.0f, fv = inside ? floorf(v) : 0.0f;
+    const float ax = inside ? u - fu : 0.0f, ay = inside ? v - fv : 0.0f;
+    const int o = (int)fv * c.w + (int)fu;
+    const float *i0 = lv.cur_int + o, *x0 = lv.cur_gx + o, *y0 = lv.cur_gy + o;
+    const float *i1 = i0 + c.w, *x1 = x0 + c.w, *y1 = y0 + c.w;
+    const float ia = __ldg(i0), ib = __ldg(i0 + 1), ic = __ldg(i1), id = __ldg(i1 + 1), ref = __ldg(lv.ref_int + k);
+    const float xa = __ldg(x0), xb = __ldg(x0 + 1), xc = __ldg(x1), xd = __ldg(x1 + 1);
+    const float ya = __ldg(y0), yb = __ldg(y0 + 1), yc = __ldg(y1), yd = __ldg(y1 + 1);
+    const float r = lerp2(ia, ib, ic, id, ax, ay) - ref;
+    const float gx = lerp2(xa, xb, xc, xd, ax, ay), gy = lerp2(ya, yb, yc, yd, ax, ay);
+    const bool ok = inside && (gx * gx + gy * gy) > 0.0f && isfinite(r);
+    res = make_float4(inside ? r : 0.0f, inside ? gx : 0.0f, inside ? gy : 0.0f, ok ? 1.0f : -1.0f);
+    if (ok) {
+        sums[0] += 1.0f;
+        sums[1] += r;
+        sums[2] += r * r;
+    }
+}
+
+// ICP half of pass A for one pixel (icp_match's decisions and products): model
+// vertex and normal loaded.  The projection uses an approximate reciprocal and
+// evaluates the exact form only where the two could round to different pixels
+// (margin: the exact form's reciprocal and products round to 3 x 2^-24, the
+// approximate ones to 2^-23 + 2 x 2^-24 relative; the sums as in integration).
+__device__ __forceinline__ float icp_margin(int n, float c) {
+    const float m = 2.0f * (float)n + fabsf(c) + 4.0f;
+    return m < 131072.0f ? 0.5f - m * 0x1p-21f : -1.0f;
+}
+__device__ __forceinline__ void fused_pixel_icp(const FusedLevel &lv, const float *T, float4 vm, float4 nm,
+                                                const IcpGates &gates, float acc[29]) {
+    const LevelCam &c = lv.c;
+    const float3 vl = make_float3(__fadd_rn(dot3_rn(T[0], T[1], T[2], vm.x, vm.y, vm.z), T[3]),
+                                  __fadd_rn(dot3_rn(T[4], T[5], T[6], vm.x, vm.y, vm.z), T[7]),
+                                  __fadd_rn(dot3_rn(T[8], T[9], T[10], vm.x, vm.y, vm.z), T[11]));
+    const float px = __fmul_rn(c.fx, vl.x), py = __fmul_rn(c.fy, vl.y), rz = rcp_approx(vl.z);
+    const float su = __fadd_rn(__fmul_rn(px, rz), c.cx), sv = __fadd_rn(__fmul_rn(py, rz), c.cy);
+    const float ku = __fadd_rn(su, 12582912.0f), kv = __fadd_rn(sv, 12582912.0f);
+    int u = __float_as_int(ku) - 0x4b400000, v = __float_as_int(kv) - 0x4b400000;
+    if (vm.w >= 0.0f && !(fabsf(__fsub_rn(su, __fsub_rn(ku, 12582912.0f))) < icp_margin(c.w, c.cx) &&
+                          fabsf(__fsub_rn(sv, __fsub_rn(kv, 12582912.0f))) < icp_margin(c.h, c.cy))) {
+        const float invz = __fdiv_rn(1.0f, vl.z);
+        const float fu = floorf(__fadd_rn(__fadd_rn(__fmul_rn(px, invz), c.cx), 0.5f));
+        const float fv = floorf(__fadd_rn(__fadd_rn(__fmul_rn(py, invz), c.cy), 0.5f));
+        u = fu >= 0.0f && fu < (float)c.w ? (int)fu : -1;
+        v = fv >= 0.0f && fv < (float)c.h ? (int)fv : -1;
+    }
+    const bool inside = vm.w >= 0.0f && (unsigned)u < (unsigned)c.w && (unsigned)v < (unsigned)c.h;
+    const int q = inside ? v * c.w + u : 0;
+    const float4 vc = __ldg(lv.cur_vmap + q), nc = __ldg(lv.cur_nmap + q);
+    const float3 nl = make_float3(dot3_rn(T[0], T[1], T[2], nm.x, nm.y, nm.z), dot3_rn(T[4], T[5], T[6], nm.x, nm.y, nm.z),
+                                  dot3_rn(T[8], T[9], T[10], nm.x, nm.y, nm.z));
+    const float dx = __fsub_rn(vl.x, vc.x), dy = __fsub_rn(vl.y, vc.y), dz = __fsub_rn(vl.z, vc.z);
+    const float ax = __fsub_rn(__fmul_rn(nc.y, nl.z), __fmul_rn(nc.z, nl.y));
+    const float ay = __fsub_rn(__fmul_rn(nc.z, nl.x), __fmul_rn(nc.x, nl.z));
+    const float az = __fsub_rn(__fmul_rn(nc.x, nl.y), __fmul_rn(nc.y, nl.x));
+    if (inside && vc.w >= 0.0f && nm.w > 0.0f && nc.w > 0.0f && dot3_rn(ax, ay, az, ax, ay, az) < gates.sin2 &&
+        dot3_rn(dx, dy, dz, dx, dy, dz) <= gates.dist2) {
+        const float r = dot3_rn(nl.x, nl.y, nl.z, __fsub_rn(vc.x, vl.x), __fsub_rn(vc.y, vl.y), __fsub_rn(vc.z, vl.z));
+        icp_accumulate(vl, nl, r, acc);
+    }
 }
 
 // Pass B for one pixel kept from pass A (gn_pass_b's products).
@@ -678,15 +736,15 @@ __device__ __forceinline__ void fused_pixel_b(const LevelCam &c, float th, const
 }
 
 
-// The CTA's row of 32 sums (warp transpose sums, then a pairwise tree over
-// the 32 warp sums of each value), published by warp 0 as tagged words.
+// The CTA's row of sums (each warp's by the transpose reduction, then a
+// pairwise tree over the warps), published by warp 0 as tagged words 0..n-1.
+// A warp without pixels (`busy` false, warp-uniform) has zero sums.
 template <int NT>
-__device__ __forceinline__ void fused_publish_row(float v[32], unsigned long long *row, unsigned tag) {
+__device__ __forceinline__ void fused_publish_row(float v[32], unsigned long long *row, unsigned tag, int n, bool busy) {
     constexpr int kFusedWarps = FoldShape<NT>::warps;
     __shared__ float wsum[kFusedWarps][33];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
-    const float r = warp_transpose_reduce(v);
-    wsum[warp][lane] = r;
+    wsum[warp][lane] = busy ? warp_transpose_reduce(v) : 0.0f;
     __syncthreads();
     if (warp == 0) {
         float x[kFusedWarps];
@@ -696,23 +754,63 @@ __device__ __forceinline__ void fused_publish_row(float v[32], unsigned long lon
         for (int s = kFusedWarps / 2; s >= 1; s >>= 1)
 #pragma unroll
             for (int i = 0; i < s; ++i) x[i] += x[i + s];
-        st_relaxed_u64(row + lane, tagged(x[0], tag));
+        if ((int)lane < n) st_relaxed_u64(row + lane, tagged(x[0], tag));
+    }
+}
+
+// The CTA's photometric moments, published as words 29..31 of its row A before
+// the ICP half of the pass, which covers their way to the other CTAs.  The sums
+// are formed as fused_publish_row forms them (a butterfly adds the same pairs).
+template <int NT>
+__device__ __forceinline__ void fused_publish_moments(float v[3], unsigned long long *row, unsigned tag, bool busy) {
+    constexpr int kFusedWarps = FoldShape<NT>::warps;
+    __shared__ float wsum[3][kFusedWarps];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    if (busy) {
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], off);
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) wsum[i][warp] = busy ? v[i] : 0.0f;
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        float x[kFusedWarps];
+#pragma unroll
+        for (int w = 0; w < kFusedWarps; ++w) x[w] = wsum[threadIdx.x][w];
+#pragma unroll
+        for (int s = kFusedWarps / 2; s >= 1; s >>= 1)
+#pragma unroll
+            for (int i = 0; i < s; ++i) x[i] += x[i + s];
+        st_relaxed_u64(row + 29 + threadIdx.x, tagged(x[0], tag));
     }
 }
 
 // Totals over all CTAs of the photometric moments (columns 29..31 of rows A)
-// into the solve's totals 29..31 of pass A; compensated FP32 per column (32
-// lanes x 5 rows, then a butterfly), kept as a double-float pair.  False on
-// abort or timeout.
+// into the solve's totals 29..31 of pass A, and the Huber threshold from them;
+// compensated FP32 per column (32 lanes x 5 rows, then a butterfly; warp 0 runs
+// the three columns side by side), kept as double-float pairs.  False on abort
+// or timeout.
+// The word that this thread folds: row r's moment q (null: none).
+__device__ __forceinline__ const unsigned long long *moment_word(const unsigned long long *rows, unsigned nrows, int &q,
+                                                                 int &r) {
+    const int t = (int)threadIdx.x, n = (int)nrows;
+    q = t >= 2 * n ? 2 : (t >= n ? 1 : 0);
+    r = t - q * n;
+    return t < 3 * n ? rows + r * 32 + 29 + q : nullptr;
+}
+// `w`: that word as it was read before the CTA published its ICP row (a first
+// poll whose way is covered by that).
 __device__ __forceinline__ bool fold_moments(const unsigned long long *rows, unsigned nrows, unsigned tag,
-                                             GNState *st, bool plain) {
+                                             GNState *st, bool plain, unsigned long long w) {
     __shared__ float m3[3][kFusedMaxCtas];
     const int t = (int)threadIdx.x;
     bool mine = true;
-    if (t < 3 * (int)nrows) {
-        const int q = t / (int)nrows, r = t - q * (int)nrows;
-        const unsigned long long *p = rows + r * 32 + 29 + q;
-        unsigned long long w = ld_relaxed_u64(p);
+    int q, r;
+    const unsigned long long *p = moment_word(rows, nrows, q, r);
+    if (p) {
         unsigned long long t0 = 0ull;
         for (unsigned spin = 0; !tag_is(w, tag); ++spin) {
             if (!poll_continue(st, spin, t0)) {
@@ -724,26 +822,36 @@ __device__ __forceinline__ bool fold_moments(const unsigned long long *rows, uns
         m3[q][r] = __uint_as_float((unsigned)w);
     }
     if (!__syncthreads_and(mine)) return false;
-    const int warp = t >> 5, lane = t & 31;
-    if (warp < 3) {
-        float h = 0.0f, l = 0.0f;
+    if (t < 32) {
+        float h[3] = {0.0f, 0.0f, 0.0f}, l[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int m = 0; m < (kFusedMaxCtas + 31) / 32; ++m) {
-            const int r = lane + 32 * m;
-            float s, e;
-            two_sum(h, r < (int)nrows ? m3[warp][r] : 0.0f, s, e);
-            h = s;
-            l += e;
+            const int r = t + 32 * m;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                float s, e;
+                two_sum(h[q], r < (int)nrows ? m3[q][r] : 0.0f, s, e);
+                h[q] = s;
+                l[q] += e;
+            }
         }
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) {
-            const float oh = __shfl_xor_sync(0xffffffffu, h, off), ol = __shfl_xor_sync(0xffffffffu, l, off);
-            float s, e;
-            two_sum(h, oh, s, e);
-            h = s;
-            l = (l + ol) + e;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const float oh = __shfl_xor_sync(0xffffffffu, h[q], off), ol = __shfl_xor_sync(0xffffffffu, l[q], off);
+                float s, e;
+                two_sum(h[q], oh, s, e);
+                h[q] = s;
+                l[q] = (l[q] + ol) + e;
+            }
         }
-        if (lane == 0) set_total(0, 29 + warp, h, plain ? 0.0f : l);
+        if (t == 0) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) set_total(0, 29 + q, h[q], plain ? 0.0f : l[q]);
+            g_solve.huber_th = huber_threshold_df(df_two(h[0], plain ? 0.0f : l[0]), df_two(h[1], plain ? 0.0f : l[1]),
+                                                  df_two(h[2], plain ? 0.0f : l[2]));
+        }
     }
     __syncthreads();
     return true;
@@ -769,15 +877,30 @@ __device__ __forceinline__ bool fold_systems(const unsigned long long *rowsA, co
     float h = 0.0f, l = 0.0f;
     if (need) {
         const unsigned long long *base = c < 32 ? rowsA + c : rowsB + (c - 32);
+        // one copy of the reads, in the loop, at 512 threads (20 rows each, and
+        // the schedule's code size counts: 206 against 208 us at 640x480); a
+        // first copy without the mask in front of it at 1024 (10 rows, 64
+        // registers: a step of eight submaps 1322 against 1343 us)
+        constexpr bool kFirstApart = NT > 512;
         unsigned long long w[kFoldRows];
+        unsigned pend = 0u;  // rows not read yet
 #pragma unroll
         for (int q = 0; q < kFoldRows; ++q) {
-            const unsigned r = (unsigned)(sub + kFoldSubsets * q);
-            w[q] = r < nrows ? ld_relaxed_u64(base + r * 32) : tagged(0.0f, tag);
+            w[q] = tagged(0.0f, tag);
+            if ((unsigned)(sub + kFoldSubsets * q) < nrows) {
+                if (kFirstApart)
+                    w[q] = ld_relaxed_u64(base + (sub + kFoldSubsets * q) * 32);
+                else
+                    pend |= 1u << q;
+            }
         }
         unsigned long long t0 = 0ull;
         for (unsigned spin = 0;; ++spin) {
-            unsigned pend = 0u;
+            if (!kFirstApart || spin != 0u)
+#pragma unroll
+                for (int q = 0; q < kFoldRows; ++q)
+                    if ((pend >> q) & 1u) w[q] = ld_relaxed_u64(base + (sub + kFoldSubsets * q) * 32);
+            pend = 0u;
 #pragma unroll
             for (int q = 0; q < kFoldRows; ++q)
                 if (!tag_is(w[q], tag)) pend |= 1u << q;
@@ -786,9 +909,6 @@ __device__ __forceinline__ bool fold_systems(const unsigned long long *rowsA, co
                 mine = false;
                 break;
             }
-#pragma unroll
-            for (int q = 0; q < kFoldRows; ++q)
-                if ((pend >> q) & 1u) w[q] = ld_relaxed_u64(base + (sub + kFoldSubsets * q) * 32);
         }
 #pragma unroll
         for (int q = 0; q < kFoldRows; ++q) {
@@ -828,14 +948,31 @@ __device__ __forceinline__ bool fold_systems(const unsigned long long *rowsA, co
 // owns at most PIX pixels per level (off = s * NT + thread, NT threads) and
 // keeps their residuals in registers for pass B; PIX == 0: any number of
 // pixels, residuals through `res4` (pass B then recomputes the warped point,
-// as gn_pass_b does), G pixels' reference loads at a time.
-template <int PIX, int NT, int G>
-__device__ __forceinline__ void gn_schedule(const FusedLevel *lvs, int L, int mode, float angle_th, float dist_th,
+// as gn_pass_b does).
+// MODE: the mode when it is known at compile time (without the tests and the
+// registers of the other modes: 640x480 RGBD 206 instead of 212 us), 0 when it
+// is `mode`.
+//
+// What bounds it: the serial chain of an iteration (moments -> threshold ->
+// pass B -> fold -> solve), of which about 7 us do not depend on the image, and
+// next to it the fetch of its instructions (65-126 KB of code, most of it run
+// once per iteration).  So the moments leave before the ICP half, whose work
+// covers their way to the other CTAs; the threshold is formed where they are
+// folded; the gathers of a thread's pixels do not branch; the ICP half gates on
+// squares and projects through an approximate reciprocal; warps without pixels
+// skip the reductions; loops keep one copy of a pixel's code and the solve's
+// rare parts are calls.  Schedules of 18 RGBD iterations before and after, with
+// the same bits: 320x240 156 / 145 us, 640x480 226 / 203, 1280x720 431 / 404; a
+// step of eight submaps 1456 / 1335.
+template <int PIX, int NT, int MODE>
+__device__ __forceinline__ void gn_schedule(const FusedLevel *lvs, int L, int mode_, IcpGates gates,
                                             unsigned long long *rows, float4 *res4, GNState *st, unsigned cta,
                                             unsigned nrows) {
     __shared__ float sRK[9];
     const int t = (int)threadIdx.x;
+    const int mode = MODE != 0 ? MODE : mode_;
     const bool do_rgb = (mode & YAS_TRACK_RGB) != 0, do_icp = (mode & YAS_TRACK_ICP) != 0;
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
     load_solve_state(st);
     if (t >= 32 && t < 64) {
         g_solve.Ah[t - 32] = 0.0f;
@@ -852,75 +989,81 @@ __device__ __forceinline__ void gn_schedule(const FusedLevel *lvs, int L, int mo
         const FusedLevel &lv = lvs[l];
         const int n = lv.c.w * lv.c.h;
         const int base = (int)cta * lv.chunk;
+        const bool busy = (t & ~31) < lv.chunk && base + (t & ~31) < n;  // the warp has pixels
+        if (t < 9) rkinv_entry(g_solve.Tf, lv.c, sRK, t);
+        __syncthreads();
         for (int it = 0; it < lv.iters; ++it) {
             ++s;
             const unsigned tag = (epoch << 12) | (s & 0xfffu);
             unsigned long long *rA = rows + (size_t)((s & 1u) * 2u + 0u) * kFusedMaxCtas * 32;
             unsigned long long *rB = rows + (size_t)((s & 1u) * 2u + 1u) * kFusedMaxCtas * 32;
-            if (t == 0) make_rkinv(g_solve.Tf, lv.c, sRK);
-            __syncthreads();
-            float acc[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
             float4 res[PIX > 0 ? PIX : 1];
             float3 pp[PIX > 0 ? PIX : 1];
-            if constexpr (PIX > 0) {
-                // the pose-independent reference loads (depth, model vertex) of
-                // every pixel first, so they are in flight together
-                float zi[PIX];
-                float4 vm[PIX];
+            float4 vm0 = none, nm0 = none;  // a single pixel's model, read ahead
+            if (PIX == 1 && do_icp && t < lv.chunk && base + t < n) {
+                vm0 = __ldg(lv.ref_vmap + base + t);
+                nm0 = __ldg(lv.ref_nmap + base + t);
+            }
+            // ---- pass A, photometric half: residuals and their moments
+            if (do_rgb) {
+                float sums[3] = {0.0f, 0.0f, 0.0f};
+                if constexpr (PIX > 0) {
+                    float zi[PIX];
 #pragma unroll
-                for (int q = 0; q < PIX; ++q) {
-                    const int off = q * NT + t;
-                    const int k = base + off;
-                    const bool own = q < lv.pix && off < lv.chunk && k < n;
-                    zi[q] = own && do_rgb ? __ldg(lv.ref_z + k) : 0.0f;
-                    vm[q] = own && do_icp ? __ldg(lv.ref_vmap + k) : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-                }
-#pragma unroll
-                for (int q = 0; q < PIX; ++q) {
-                    res[q] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-                    pp[q] = make_float3(0.0f, 0.0f, 1.0f);
-                    const int off = q * NT + t;
-                    const int k = base + off;
-                    if (q < lv.pix && off < lv.chunk && k < n)
-                        fused_pixel_a_pre(lv, g_solve.Tf, sRK, k, do_rgb, do_icp, angle_th, dist_th, zi[q], vm[q], acc,
-                                          res[q], pp[q]);
-                }
-            } else {
-                // pixels off = t, t + NT, ... in groups of G, each group's
-                // reference loads first (the same pixels in the same order as
-                // one at a time); G = 2 in the batched schedules, whose CTAs
-                // own tens of pixels per thread, G = 1 where a second
-                // pixel's registers would spill (1024 threads, 64 registers)
-#pragma unroll 1
-                for (int off0 = t; off0 < lv.chunk; off0 += G * NT) {
-                    float zi[G];
-                    float4 vm[G];
-#pragma unroll
-                    for (int q = 0; q < G; ++q) {
-                        const int off = off0 + q * NT, k = base + off;
-                        const bool own = off < lv.chunk && k < n;
-                        zi[q] = own && do_rgb ? __ldg(lv.ref_z + k) : 0.0f;
-                        vm[q] = own && do_icp ? __ldg(lv.ref_vmap + k) : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+                    for (int q = 0; q < PIX; ++q) {
+                        const int off = q * NT + t, k = base + off;
+                        zi[q] = q < lv.pix && off < lv.chunk && k < n ? __ldg(lv.ref_z + k) : 0.0f;
                     }
 #pragma unroll
-                    for (int q = 0; q < G; ++q) {
-                        const int off = off0 + q * NT, k = base + off;
-                        if (off >= lv.chunk || k >= n) break;
+                    for (int q = 0; q < PIX; ++q) {
+                        res[q] = none;
+                        pp[q] = make_float3(0.0f, 0.0f, 1.0f);
+                        const int off = q * NT + t, k = base + off;
+                        if (q < lv.pix && off < lv.chunk && k < n)
+                            fused_pixel_rgb(lv, g_solve.Tf, sRK, k, zi[q], sums, res[q], pp[q]);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int off = t; off < lv.chunk; off += NT) {
+                        const int k = base + off;
+                        if (k >= n) break;
                         float4 r4;
                         float3 p3;
-                        fused_pixel_a_pre(lv, g_solve.Tf, sRK, k, do_rgb, do_icp, angle_th, dist_th, zi[q], vm[q], acc,
-                                          r4, p3);
-                        if (do_rgb) res4[k] = r4;
+                        fused_pixel_rgb(lv, g_solve.Tf, sRK, k, __ldg(lv.ref_z + k), sums, r4, p3);
+                        res4[k] = r4;
                     }
                 }
+                fused_publish_moments<NT>(sums, rA + cta * 32, tag, busy);
             }
-            fused_publish_row<NT>(acc, rA + cta * 32, tag);
+            float acc[32];
+            int mq, mr;
+            const unsigned long long *mword = do_rgb ? moment_word(rA, nrows, mq, mr) : nullptr;
+            unsigned long long mw = 0ull;
+            // ---- pass A, ICP half
+            if (do_icp) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
+                if constexpr (PIX == 1) {
+                    const int k = base + t;
+                    if (t < lv.chunk && k < n) fused_pixel_icp(lv, g_solve.Tf, vm0, nm0, gates, acc);
+                } else {
+                    // one copy of the pixel's code: the schedule's size counts
+                    // (640x480: 203 us, unrolled with the vertices read ahead 205)
+#pragma unroll 1
+                    for (int off = t; off < lv.chunk; off += NT) {
+                        const int k = base + off;
+                        if (k >= n) break;
+                        fused_pixel_icp(lv, g_solve.Tf, __ldg(lv.ref_vmap + k), __ldg(lv.ref_nmap + k), gates, acc);
+                    }
+                }
+                if (mword) mw = ld_relaxed_u64(mword);
+                fused_publish_row<NT>(acc, rA + cta * 32, tag, 29, busy);
+            } else if (mword) {
+                mw = ld_relaxed_u64(mword);
+            }
             if (do_rgb) {
-                if (!fold_moments(rA, nrows, tag, st, plain)) return;
-                if (t == 0) g_solve.huber_th = huber_threshold_solve();
-                __syncthreads();
+                // ---- pass B: weighted photometric products
+                if (!fold_moments(rA, nrows, tag, st, plain, mw)) return;
                 const float th = g_solve.huber_th;
 #pragma unroll
                 for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
@@ -930,36 +1073,28 @@ __device__ __forceinline__ void gn_schedule(const FusedLevel *lvs, int L, int mo
                         if (res[q].w > 0.0f) fused_pixel_b(lv.c, th, res[q], pp[q], acc);
                 } else {
 #pragma unroll 1
-                    for (int off0 = t; off0 < lv.chunk; off0 += G * NT) {
-                        float4 r4[G];
-                        float zi[G];
-#pragma unroll
-                        for (int q = 0; q < G; ++q) {
-                            const int off = off0 + q * NT, k = base + off;
-                            const bool own = off < lv.chunk && k < n;
-                            r4[q] = own ? res4[k] : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-                            zi[q] = own ? __ldg(lv.ref_z + k) : 1.0f;
-                        }
-#pragma unroll
-                        for (int q = 0; q < G; ++q) {
-                            const int k = base + off0 + q * NT;
-                            if (r4[q].w > 0.0f) {
-                                const int y = k / lv.c.w, x = k - y * lv.c.w;
-                                const float3 p3 = warp_ref_point(sRK, g_solve.Tf, x, y, zi[q]);
-                                fused_pixel_b(lv.c, th, r4[q], p3, acc);
-                            }
+                    for (int off = t; off < lv.chunk; off += NT) {
+                        const int k = base + off;
+                        if (k >= n) break;
+                        const float4 r4 = res4[k];
+                        if (r4.w > 0.0f) {
+                            int x, y;
+                            pixel_of(lv, k, x, y);
+                            const float3 p3 = warp_ref_point(sRK, g_solve.Tf, x, y, __ldg(lv.ref_z + k));
+                            fused_pixel_b(lv.c, th, r4, p3, acc);
                         }
                     }
                 }
-                fused_publish_row<NT>(acc, rB + cta * 32, tag);
+                fused_publish_row<NT>(acc, rB + cta * 32, tag, 28, busy);
             }
             if (!fold_systems<NT>(rA, rB, nrows, tag, do_icp, do_rgb, st, plain)) return;
             if (t < 32) {
                 if (!do_rgb && t == 0) g_solve.huber_th = huber_threshold_solve();
                 if constexpr (NT <= 512)
-                    gn_solve_inline(mode, 0, it == 0, l);
+                    gn_solve_inline<true>(mode, 0, it == 0, l);
                 else
                     gn_solve(mode, 0, it == 0, l);
+                if (do_rgb && t < 9) rkinv_entry(g_solve.Tf, lv.c, sRK, t);  // of the level's next iteration
             }
             __syncthreads();
             if (g_solve.failed != 0) {
@@ -976,9 +1111,9 @@ __device__ __forceinline__ void gn_schedule(const FusedLevel *lvs, int L, int mo
 }
 
 // The fused schedule of one tracker over the whole grid.
-template <int PIX>
+template <int PIX, int MODE>
 __global__ void __launch_bounds__(fused_threads<PIX>(), 1) gn_fused(const __grid_constant__ FusedArgs a) {
-    gn_schedule<PIX, fused_threads<PIX>(), 1>(a.lv, a.L, a.mode, a.angle_th, a.dist_th, a.rows, a.res4, a.st, blockIdx.x, gridDim.x);
+    gn_schedule<PIX, fused_threads<PIX>(), MODE>(a.lv, a.L, a.mode, a.gates, a.rows, a.res4, a.st, blockIdx.x, gridDim.x);
 }
 
 // Fused schedules of a batch of trackers in one launch: CTA b runs for item
@@ -986,11 +1121,12 @@ __global__ void __launch_bounds__(fused_threads<PIX>(), 1) gn_fused(const __grid
 // so an item's result is the same alone and in any batch.
 // PIX > 0: every item's CTAs own at most PIX pixels per thread on every level
 // (residuals kept in registers); PIX == 0: any share (residuals in res4).
-template <int PIX>
+// MODE: the items' common mode, 0 for items of several modes.
+template <int PIX, int MODE>
 __global__ void __launch_bounds__(kBatchThreads, 1) gn_fused_batch(const GNBatchItem *__restrict__ items,
                                                                     const unsigned short *__restrict__ cta_item) {
     const GNBatchItem &it = items[cta_item[blockIdx.x]];
-    gn_schedule<PIX, kBatchThreads, 2>(it.lv, it.L, it.mode, it.angle_th, it.dist_th, it.rows, it.res4, it.st,
+    gn_schedule<PIX, kBatchThreads, MODE>(it.lv, it.L, it.mode, it.gates, it.rows, it.res4, it.st,
                                     blockIdx.x - (unsigned)it.cta0, (unsigned)it.nctas);
 }
 
@@ -1056,8 +1192,8 @@ void launch_gn_iteration(yas_tracker *tr, int l, bool first_of_level, cudaStream
 }
 
 
-template <int PIX>
-static cudaError_t launch_fused_pix(const FusedArgs &a, int grid, cudaStream_t s) {
+template <int PIX, int MODE>
+static cudaError_t launch_fused_mode(const FusedArgs &a, int grid, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(fused_threads<PIX>());
@@ -1068,7 +1204,14 @@ static cudaError_t launch_fused_pix(const FusedArgs &a, int grid, cudaStream_t s
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gn_fused<PIX>, a);
+    return cudaLaunchKernelEx(&cfg, gn_fused<PIX, MODE>, a);
+}
+
+template <int PIX>
+static cudaError_t launch_fused_pix(const FusedArgs &a, int grid, cudaStream_t s) {
+    return a.mode == YAS_TRACK_RGBD  ? launch_fused_mode<PIX, YAS_TRACK_RGBD>(a, grid, s)
+           : a.mode == YAS_TRACK_ICP ? launch_fused_mode<PIX, YAS_TRACK_ICP>(a, grid, s)
+                                     : launch_fused_mode<PIX, YAS_TRACK_RGB>(a, grid, s);
 }
 
 // Grid of the fused schedule: one CTA per SM (512 threads; 1024 for PIX = 0),
@@ -1084,10 +1227,22 @@ static bool fused_plan(yas_tracker *tr, int &pix, int &grid) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
         int nb[4] = {0, 0, 0, 0};
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[0], gn_fused<1>, fused_threads<1>(), 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[1], gn_fused<2>, fused_threads<2>(), 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[2], gn_fused<4>, fused_threads<4>(), 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[3], gn_fused<0>, fused_threads<0>(), 0);
+        // of the mode's own kernels
+        const auto resident = [&](auto k1, auto k2, auto k4, auto k0) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[0], k1, fused_threads<1>(), 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[1], k2, fused_threads<2>(), 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[2], k4, fused_threads<4>(), 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[3], k0, fused_threads<0>(), 0);
+        };
+        if (tr->mode == YAS_TRACK_RGBD)
+            resident(gn_fused<1, YAS_TRACK_RGBD>, gn_fused<2, YAS_TRACK_RGBD>, gn_fused<4, YAS_TRACK_RGBD>,
+                     gn_fused<0, YAS_TRACK_RGBD>);
+        else if (tr->mode == YAS_TRACK_ICP)
+            resident(gn_fused<1, YAS_TRACK_ICP>, gn_fused<2, YAS_TRACK_ICP>, gn_fused<4, YAS_TRACK_ICP>,
+                     gn_fused<0, YAS_TRACK_ICP>);
+        else
+            resident(gn_fused<1, YAS_TRACK_RGB>, gn_fused<2, YAS_TRACK_RGB>, gn_fused<4, YAS_TRACK_RGB>,
+                     gn_fused<0, YAS_TRACK_RGB>);
         cudaGetLastError();
         // one CTA per SM (the schedule's design), whatever else would fit
         for (int i = 0; i < 4; ++i)
@@ -1114,12 +1269,25 @@ static bool fused_plan(yas_tracker *tr, int &pix, int &grid) {
     return false;
 }
 
+// Thresholds are positive and finite.
+static IcpGates icp_gates(float angle_th, float dist_th) {
+    IcpGates g;
+    g.dist2 = dist_th * dist_th;
+    while (sqrtf(nextafterf(g.dist2, INFINITY)) <= dist_th) g.dist2 = nextafterf(g.dist2, INFINITY);
+    while (sqrtf(g.dist2) > dist_th) g.dist2 = nextafterf(g.dist2, 0.0f);
+    g.sin2 = angle_th * angle_th;
+    while (sqrtf(g.sin2) < angle_th) g.sin2 = nextafterf(g.sin2, INFINITY);
+    while (g.sin2 > 0.0f && !(sqrtf(nextafterf(g.sin2, 0.0f)) < angle_th)) g.sin2 = nextafterf(g.sin2, 0.0f);
+    return g;
+}
+
 // Levels of a fused schedule run by `grid` CTAs, on the tracker's current sets.
 static void fill_levels(yas_tracker *tr, int grid, int threads, FusedLevel *lv) {
     for (int l = 0; l < tr->L; ++l) {
         FusedLevel &f = lv[l];
         f.c = tr->cam[l];
         f.iters = tr->iters[l];
+        f.wdiv = (unsigned)(((1ull << 32) + (unsigned)f.c.w - 1u) / (unsigned)f.c.w);
         const long long P = (long long)f.c.w * f.c.h;
         f.chunk = (int)(((P + grid - 1) / grid + 31) / 32 * 32);
         f.pix = (f.chunk + threads - 1) / threads;
@@ -1145,8 +1313,7 @@ static bool launch_gn_fused(yas_tracker *tr, cudaStream_t s) {
     fill_levels(tr, grid, pix == 0 ? fused_threads<0>() : fused_threads<1>(), a.lv);
     a.L = tr->L;
     a.mode = tr->mode;
-    a.angle_th = tr->angle_th;
-    a.dist_th = tr->dist_th;
+    a.gates = icp_gates(tr->angle_th, tr->dist_th);
     a.rows = tr->fused_rows;
     a.res4 = tr->res4;
     a.st = tr->state;
@@ -1184,8 +1351,7 @@ void gn_batch_item_ctas(yas_tracker *tr, int cta0, int nctas, GNBatchItem *out) 
     fill_levels(tr, out->nctas, kBatchThreads, out->lv);
     out->L = tr->L;
     out->mode = tr->mode;
-    out->angle_th = tr->angle_th;
-    out->dist_th = tr->dist_th;
+    out->gates = icp_gates(tr->angle_th, tr->dist_th);
     out->rows = tr->fused_rows;
     out->res4 = tr->res4;
     out->st = tr->state;
@@ -1201,7 +1367,9 @@ int gn_batch_capacity() {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
         int lowest = 1 << 30;
-        for (auto k : {gn_fused_batch<0>, gn_fused_batch<1>, gn_fused_batch<2>, gn_fused_batch<4>}) {
+        for (auto k : {gn_fused_batch<0, 0>, gn_fused_batch<1, 0>, gn_fused_batch<2, 0>, gn_fused_batch<4, 0>,
+                       gn_fused_batch<0, YAS_TRACK_RGBD>, gn_fused_batch<1, YAS_TRACK_RGBD>,
+                       gn_fused_batch<2, YAS_TRACK_RGBD>, gn_fused_batch<4, YAS_TRACK_RGBD>}) {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kBatchThreads, 0);
             lowest = std::min(lowest, nb);
         }
@@ -1211,15 +1379,18 @@ int gn_batch_capacity() {
     return cap[dev];
 }
 
-int gn_batch_pix(const GNBatchItem *items, int n) {
-    int pix = 0;
-    for (int i = 0; i < n; ++i)
+GNBatchShape gn_batch_shape(const GNBatchItem *items, int n) {
+    int pix = 0, mode = n > 0 ? items[0].mode : 0;
+    for (int i = 0; i < n; ++i) {
+        if (items[i].mode != mode) mode = 0;
         for (int l = 0; l < items[i].L; ++l) pix = std::max(pix, items[i].lv[l].pix);
-    return pix <= 1 ? 1 : (pix <= 2 ? 2 : (pix <= 4 ? 4 : 0));
+    }
+    // the RGB+ICP mode has kernels of its own; others, and mixed batches, share
+    return GNBatchShape{pix <= 1 ? 1 : (pix <= 2 ? 2 : (pix <= 4 ? 4 : 0)), mode == YAS_TRACK_RGBD ? mode : 0};
 }
 
 cudaError_t launch_gn_batch(const GNBatchItem *dev_items, const unsigned short *dev_cta_item, int grid,
-                            cudaStream_t s, int pix) {
+                            cudaStream_t s, GNBatchShape shape) {
     if (grid <= 0 || grid > gn_batch_capacity()) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -1230,11 +1401,14 @@ cudaError_t launch_gn_batch(const GNBatchItem *dev_items, const unsigned short *
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    switch (pix) {
-        case 1: return cudaLaunchKernelEx(&cfg, gn_fused_batch<1>, dev_items, dev_cta_item);
-        case 2: return cudaLaunchKernelEx(&cfg, gn_fused_batch<2>, dev_items, dev_cta_item);
-        case 4: return cudaLaunchKernelEx(&cfg, gn_fused_batch<4>, dev_items, dev_cta_item);
-        default: return cudaLaunchKernelEx(&cfg, gn_fused_batch<0>, dev_items, dev_cta_item);
+    const auto launch = [&](auto rgbd, auto any) {
+        return cudaLaunchKernelEx(&cfg, shape.mode == YAS_TRACK_RGBD ? rgbd : any, dev_items, dev_cta_item);
+    };
+    switch (shape.pix) {
+        case 1: return launch(gn_fused_batch<1, YAS_TRACK_RGBD>, gn_fused_batch<1, 0>);
+        case 2: return launch(gn_fused_batch<2, YAS_TRACK_RGBD>, gn_fused_batch<2, 0>);
+        case 4: return launch(gn_fused_batch<4, YAS_TRACK_RGBD>, gn_fused_batch<4, 0>);
+        default: return launch(gn_fused_batch<0, YAS_TRACK_RGBD>, gn_fused_batch<0, 0>);
     }
 }
 

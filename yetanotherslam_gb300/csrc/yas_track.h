@@ -49,6 +49,14 @@ struct __align__(16) GNState {
     unsigned plain_sums;    // 1: plain FP32 totals (the reference's); 0: compensated totals
 };
 
+// ICP gates of a launch: the largest squared distance and the smallest squared
+// sine whose rounded square root fails the test against the threshold.  The
+// square root is monotone, so comparing its argument takes the same decisions.
+struct IcpGates {
+    float dist2;  // |v_m - v_c| <= dist_th  <=>  its square <= dist2
+    float sin2;   // |n_c x n_m| < angle_th  <=>  its square < sin2
+};
+
 // One pyramid level of a fused Gauss-Newton schedule: camera, iterations,
 // the pixel share of each CTA and the level maps.
 struct FusedLevel {
@@ -56,6 +64,7 @@ struct FusedLevel {
     int iters;
     int chunk;  // pixels per CTA (a multiple of 32)
     int pix;    // pixels per thread, ceil(chunk / threads per CTA)
+    unsigned wdiv;  // ceil(2^32 / width)
     const float *ref_int, *ref_invd, *ref_z;
     const float4 *ref_vmap, *ref_nmap;
     const float *cur_int, *cur_gx, *cur_gy;
@@ -67,7 +76,7 @@ struct FusedLevel {
 struct GNBatchItem {
     FusedLevel lv[kMaxLevels];
     int L, mode;
-    float angle_th, dist_th;
+    IcpGates gates;
     unsigned long long *rows;
     float4 *res4;
     GNState *st;
@@ -156,10 +165,13 @@ int gn_batch_ctas(const yas_tracker *tr, int pixels_per_cta = 32768);
 void gn_batch_item(yas_tracker *tr, int cta0, GNBatchItem *out, int pixels_per_cta = 32768);
 // the same with an explicit CTA count (1..kFusedMaxCtas)
 void gn_batch_item_ctas(yas_tracker *tr, int cta0, int nctas, GNBatchItem *out);
-// the batched kernel's pixels-per-thread variant for these (host) descriptors:
-// 1, 2, 4 (residuals in registers) or 0 (any share)
-int gn_batch_pix(const GNBatchItem *items, int n);
+// the batched kernel's variant for these (host) descriptors: pixels per thread
+// 1, 2, 4 (residuals in registers) or 0 (any share), and their common mode
+struct GNBatchShape {
+    int pix, mode;
+};
+GNBatchShape gn_batch_shape(const GNBatchItem *items, int n);
 int gn_batch_capacity();                                // co-resident CTAs of the batched launch
 cudaError_t launch_gn_batch(const GNBatchItem *dev_items, const unsigned short *dev_cta_item, int grid,
-                            cudaStream_t s, int pix);
+                            cudaStream_t s, GNBatchShape shape);
 }  // namespace yas
