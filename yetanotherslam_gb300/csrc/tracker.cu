@@ -1479,30 +1479,17 @@ void tracker_free(yas_tracker *tr) {
 void tracker_image(yas_tracker *tr, const uint8_t *src, int channels, int pitch, bool reference,
                    cudaStream_t s) {
     TrackLevelBufs *B = reference ? tr->set[1 - tr->cur] : tr->set[tr->cur];
-    // The reference set has no gradient maps: write them to the current-frame
-    // gradient buffers only when preparing the current frame.
-    float *gx0 = reference ? nullptr : tr->gx[0];
-    float *gy0 = reference ? nullptr : tr->gy[0];
-    if (reference) {
-        // gradients of a reference image are not used; compute into res4 scratch
-        gx0 = reinterpret_cast<float *>(tr->res4);
-        gy0 = gx0 + (size_t)tr->w * tr->h;
-    }
-    launch_image_level0(src, channels, 0, pitch, tr->w, tr->h, B[0].intensity, gx0, gy0, s);
-    for (int l = 1; l < tr->L; ++l)
-        launch_image_level(B[l - 1].intensity, tr->cam[l - 1].w, tr->cam[l - 1].h, tr->cam[l].w,
-                           tr->cam[l].h, B[l].intensity, reference ? nullptr : tr->gx[l],
-                           reference ? nullptr : tr->gy[l], s);
+    float *inten[kMaxLevels];
+    for (int l = 0; l < tr->L; ++l) inten[l] = B[l].intensity;
+    // the reference set has no gradient maps
+    launch_image_pyramid(src, channels, pitch, tr->L, tr->cam, inten, reference ? nullptr : tr->gx,
+                         reference ? nullptr : tr->gy, s);
 }
 
 void tracker_depth(yas_tracker *tr, const void *src, int is_u16, int pitch, float scale, float *depth_m,
                    bool reference, cudaStream_t s) {
     TrackLevelBufs *B = reference ? tr->set[1 - tr->cur] : tr->set[tr->cur];
-    launch_depth_level0(src, is_u16, pitch, scale, tr->cam[0], depth_m, B[0].invd, B[0].z, B[0].vmap, B[0].nmap,
-                        s);
-    for (int l = 1; l < tr->L; ++l)
-        launch_depth_level(B[l - 1].invd, tr->cam[l - 1].w, tr->cam[l], B[l].invd, B[l].z, B[l].vmap, B[l].nmap,
-                           s);
+    launch_depth_pyramid(src, is_u16, pitch, scale, tr->L, tr->cam, depth_m, B, s);
 }
 
 void tracker_model(yas_tracker *tr, cudaStream_t s) {

@@ -91,14 +91,10 @@ struct TrackLevelBufs {
     float4 *nmap;
 };
 
-void launch_image_level0(const uint8_t *src, int channels, int bgr, int pitch, int w, int h, float *inten,
-                         float *gx, float *gy, cudaStream_t s);
-void launch_image_level(const float *prev, int pw, int ph, int w, int h, float *inten, float *gx, float *gy,
-                        cudaStream_t s);
-void launch_depth_level0(const void *src, int is_u16, int pitch, float scale, const LevelCam &c,
-                         float *depth_m, float *invd, float *zmap, float4 *vmap, float4 *nmap, cudaStream_t s);
-void launch_depth_level(const float *prev, int pw, const LevelCam &c, float *invd, float *zmap, float4 *vmap,
-                        float4 *nmap, cudaStream_t s);
+void launch_image_pyramid(const uint8_t *src, int channels, int pitch, int L, const LevelCam *cam,
+                          float *const *inten, float *const *gx, float *const *gy, cudaStream_t s);
+void launch_depth_pyramid(const void *src, int is_u16, int pitch, float scale, int L, const LevelCam *cam,
+                          float *depth_m, TrackLevelBufs *out, cudaStream_t s);
 void launch_model_pyramid(int L, const int *w, const int *h, float4 *const *vmap, float4 *const *nmap,
                           cudaStream_t s);
 void launch_render_scene(const float4 *vmap, const float4 *nmap, int vpitch, int w, int h, float3 light,
