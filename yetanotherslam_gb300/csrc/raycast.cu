@@ -20,8 +20,19 @@
 // 4- or 8-byte load each.  Per raycast (warm, events around the kernel; before:
 // hash lookups, image order, 32 rays a warp): 640x480, 5 mm F16 122 -> 79 us,
 // 1280x720, 4 mm F16 241 -> 166, 320x240, 8 mm F32 77 -> 50, 160x120, 1 cm F32
-// 72 -> 38.  What is left is instruction issue in large images (60% of the
-// slots; 20 of 32 lanes active) and the chain of the longest rays in small ones.
+// 72 -> 38.  A map that has been tracked against for long takes more: its rays
+// cross the layers that drift left (at 640x480, 5 mm after 1000 frames 38
+// samples a ray instead of 11, 10 of them interpolated).  There the warps are
+// bound by the instructions of an iteration, whose lanes look up, jump and
+// interpolate in turn (14 of 32 active, 65% of the issue slots), and the last by
+// the chain of the longest rays; floors without conversion instructions, the
+// neighbours of a cell read side by side, and packed lerps take such a raycast
+// (its other kernels included) from 264 to 218 us, a new map's from 115 to 109,
+// 1280x720, 4 mm after 600 frames from 420 to 371.  Not kept: interpolated samples
+// handed round the warp four lanes each (242 us), steps until most lanes
+// interpolate (286 and more), 16 or 8 rays a warp for the long ones (262, 329),
+// tiles in the order of the last raycast's sample counts (213, but 91 instead
+// of 84 us at 320x240).
 // Deliberate differences: a missed ray writes w = -1 (the reference leaves w
 // stale on its early return, RayTraceEngine.cu:338-347); the 8 trilinear
 // corners are floor(p) + {0,1}^3 (the reference floors p + offset per corner).
@@ -230,6 +241,32 @@ void launch_block_grid(const MapDev &m, const PosePair *P, const RaycastBuffers 
     grid_fill_kernel<<<kSMs, 256, 0, s>>>(m, rb.grid);
 }
 
+// floor(x) and its integer.  NEAR: |x| < 2^22, by one sum rounded down (the
+// conversion instructions run at a quarter of the rate).
+constexpr float kFloorShift = 12582912.0f;  // 1.5 x 2^23
+template <bool NEAR>
+__device__ __forceinline__ float floor_of(float x, int &i) {
+    if (NEAR) {
+        const float k = __fadd_rd(x, kFloorShift);
+        i = __float_as_int(k) - 0x4b400000;
+        return __fsub_rn(k, kFloorShift);
+    }
+    const float f = floorf(x);
+    i = (int)f;
+    return f;
+}
+template <bool NEAR>
+__device__ __forceinline__ int ifloor_of(float x) {
+    int i;
+    floor_of<NEAR>(x, i);
+    return i;
+}
+
+// The reference's lerp (1 - t) a + t b of a pair.
+__device__ __forceinline__ float2 mix2(float2 a, float2 b, float t) {
+    return cfma2(pair(1.0f - t), a, cmul2(pair(t), b));
+}
+
 // Reads of one ray.
 template <int FMT>
 struct RayReader {
@@ -267,42 +304,63 @@ struct RayReader {
         return IO::sdf(v);
     }
     // Trilinear sample at p, whose block (bx, by, bz) has pool index b, with the
-    // reference's lerp order (RayTraceEngine.cu:297-329).  A third of the 2x2x2
-    // cells straddle a block face: their lanes look the neighbours up (1, 3 or
-    // 7 of them, the submasks d of the straddled axes; corner c lies in
-    // neighbour c & across), then every lane reads its eight corners.
+    // reference's lerp order (RayTraceEngine.cu:297-329).  Corner c of the 2x2x2
+    // cell lies in neighbour c & across, across the set of axes on which the cell
+    // straddles a block face (a third of the cells straddle one): their lanes read
+    // the seven corners' grid words side by side; only at the grid's border, or
+    // for a block that the grid leaves to the table, they look up one by one.
+    template <bool NEAR>
     __device__ __forceinline__ float interp(float3 p, int bx, int by, int bz, int b, bool &valid) const {
-        const float fx = floorf(p.x), fy = floorf(p.y), fz = floorf(p.z);
-        const int x0 = (int)fx, y0 = (int)fy, z0 = (int)fz;
-        const float ax = p.x - fx, ay = p.y - fy, az = p.z - fz;
+        int x0, y0, z0;
+        const float ax = p.x - floor_of<NEAR>(p.x, x0), ay = p.y - floor_of<NEAR>(p.y, y0);
+        const float az = p.z - floor_of<NEAR>(p.z, z0);
         const unsigned across = ((x0 & 7) == 7 ? 1u : 0u) | ((y0 & 7) == 7 ? 2u : 0u) | ((z0 & 7) == 7 ? 4u : 0u);
-        int q[8];  // pool index of each corner's block
+        unsigned q[8], lim = 0x80000000u;  // pool index of each corner's block (lim or above: unallocated)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) q[c] = b;
-        for (unsigned d = across; d != 0u; d = (d - 1u) & across) {
-            const int e = lookup(bx + (int)(d & 1u), by + (int)((d >> 1) & 1u), bz + (int)(d >> 2));
+        for (int c = 0; c < 8; ++c) q[c] = (unsigned)b;
+        if (across != 0u) {
+            const int gx = bx - ox, gy = by - oy, gz = bz - oz;
+            bool ask = true;
+            lim = kGridAsk;
+            if (max(max((unsigned)gx, (unsigned)gy), (unsigned)gz) < (unsigned)(kGridSide - 1)) {
+                const unsigned *cell = g.cells + grid_cell(gx, gy, gz);
+                const int sx = across & 1u, sy = across & 2u ? kGridSide : 0, sz = across & 4u ? kGridSide * kGridSide : 0;
+                ask = false;
 #pragma unroll
-            for (unsigned c = 1u; c < 8u; ++c) q[c] = (c & across) == d ? e : q[c];
+                for (int c = 1; c < 8; ++c) {
+                    q[c] = __ldg(cell + ((c & 1 ? sx : 0) + (c & 2 ? sy : 0) + (c & 4 ? sz : 0))) - epoch;
+                    ask = ask || q[c] == kGridAsk;
+                }
+            }
+            if (ask) {
+                lim = 0x80000000u;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) q[c] = (unsigned)b;
+#pragma unroll 1
+                for (unsigned d = across; d != 0u; d = (d - 1u) & across) {
+                    const int e = lookup(bx + (int)(d & 1u), by + (int)((d >> 1) & 1u), bz + (int)(d >> 2));
+#pragma unroll
+                    for (unsigned c = 1u; c < 8u; ++c) q[c] = (c & across) == d ? (unsigned)e : q[c];
+                }
+            }
         }
         const int xo[2] = {x0 & 7, (x0 + 1) & 7}, yo[2] = {(y0 & 7) << 3, ((y0 + 1) & 7) << 3};
         const int zo[2] = {(z0 & 7) << 6, ((z0 + 1) & 7) << 6};
         V v[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c)
-            v[c] = q[c] >= 0 ? __ldg(vox + (size_t)q[c] * kBlockVoxels + (zo[c >> 2] + yo[(c >> 1) & 1] + xo[c & 1]))
-                             : IO::make(1.0f, 0);
+            v[c] = q[c] < lim ? __ldg(vox + (size_t)q[c] * kBlockVoxels + (zo[c >> 2] + yo[(c >> 1) & 1] + xo[c & 1]))
+                                : IO::make(1.0f, 0);
         bool ok = true;
         float s[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) s[c] = value(v[c], ok);
-        float r0 = (1.0f - ax) * s[0] + ax * s[1];
-        float r1 = (1.0f - ax) * s[2] + ax * s[3];
-        const float r2 = (1.0f - ay) * r0 + ay * r1;
-        r0 = (1.0f - ax) * s[4] + ax * s[5];
-        r1 = (1.0f - ax) * s[6] + ax * s[7];
-        const float r3 = (1.0f - ay) * r0 + ay * r1;
         valid = ok;
-        return (1.0f - az) * r2 + az * r3;
+        // two at a time: the upper and lower plane side by side
+        const float2 r0 = mix2(make_float2(s[0], s[4]), make_float2(s[1], s[5]), ax);
+        const float2 r1 = mix2(make_float2(s[2], s[6]), make_float2(s[3], s[7]), ax);
+        const float2 r2 = mix2(r0, r1, ay);
+        return fmaf(1.0f - az, r2.x, __fmul_rn(az, r2.y));
     }
 };
 
@@ -349,16 +407,30 @@ __device__ __forceinline__ bool ray_setup(const Cam &cam, const Rigid32 &T, floa
     return true;
 }
 
+// Every sample of the march lies within 2^22 voxels of the origin (no NaN).
+__device__ __forceinline__ bool ray_near(const RayState &R) {
+    return fabsf(R.r.x) < 2097152.0f && fabsf(R.r.y) < 2097152.0f && fabsf(R.r.z) < 2097152.0f &&
+           R.dist_e - R.dist_s < 1048576.0f && R.dir.x + R.dir.y + R.dir.z < 4.0f;
+}
+
+// R.r n steps on.
+__device__ __forceinline__ float3 at_step(const RayState &R, float n) {
+    const float2 xy = cfma2(pair(n), make_float2(R.dir.x, R.dir.y), make_float2(R.r.x, R.r.y));
+    return make_float3(xy.x, xy.y, fmaf(n, R.dir.z, R.r.z));
+}
+
 // One axis of a ray in an unallocated block whose lower face is at x0.  `face`
 // is the face that the ray leaves through (1e30 for a ray parallel to the
 // axis: none); the result is the steps to the first sample at or past it (the
-// upper face is outside the block, the lower one inside).  idir is -1 / dir
-// for a rising ray, 1 / dir for a falling one, 1 for a parallel one.
+// upper face is outside the block, the lower one inside): the quotient rounded
+// up for a rising ray, the next whole number above it for a falling one.  idir
+// is -1 / |dir| (1 for a parallel ray): a rising ray's quotient is negative.
+template <bool NEAR>
 __device__ __forceinline__ float exit_steps(float x0, float r, float dir, float idir, float &face) {
     const bool falls = dir < 0.0f;
     face = x0 + (falls ? 0.0f : (dir > 0.0f ? 8.0f : 1e30f));
-    const float t = floorf((face - r) * idir);
-    return falls ? t + 1.0f : (dir > 0.0f ? -t : 1e30f);
+    const float u = (face - r) * idir;
+    return fabsf(NEAR ? __fsub_rn(__fadd_rd(u, kFloorShift), kFloorShift) : floorf(u)) + (falls ? 1.0f : 0.0f);
 }
 // p is outside the block on that axis (it came from inside along dir).
 __device__ __forceinline__ bool past(float p, float dir, float face) { return (p >= face) != (dir < 0.0f); }
@@ -370,28 +442,29 @@ __device__ __forceinline__ bool past(float p, float dir, float face) { return (p
 // sample k - 1 (computed as the move computes it) is still in the block and
 // sample k is not, the move goes straight to sample k; otherwise (k rounded
 // the wrong way) it keeps two samples as margin, at least one step.
+template <bool NEAR>
 __device__ __forceinline__ float empty_steps(const RayState &R, float x0, float y0, float z0) {
     float fx, fy, fz;
-    const float kx = exit_steps(x0, R.r.x, R.dir.x, R.idir.x, fx), ky = exit_steps(y0, R.r.y, R.dir.y, R.idir.y, fy);
-    const float kz = exit_steps(z0, R.r.z, R.dir.z, R.idir.z, fz);
-    const float k = fminf(fminf(kx, ky), kz), a = k - 1.0f;
-    const bool in = !(past(R.r.x + a * R.dir.x, R.dir.x, fx) || past(R.r.y + a * R.dir.y, R.dir.y, fy) ||
-                      past(R.r.z + a * R.dir.z, R.dir.z, fz));
-    const bool out = past(R.r.x + k * R.dir.x, R.dir.x, fx) || past(R.r.y + k * R.dir.y, R.dir.y, fy) ||
-                     past(R.r.z + k * R.dir.z, R.dir.z, fz);
+    const float kx = exit_steps<NEAR>(x0, R.r.x, R.dir.x, R.idir.x, fx), ky = exit_steps<NEAR>(y0, R.r.y, R.dir.y, R.idir.y, fy);
+    const float kz = exit_steps<NEAR>(z0, R.r.z, R.dir.z, R.idir.z, fz);
+    const float k = fminf(fminf(kx, ky), kz);
+    const float3 p = at_step(R, k - 1.0f), q = at_step(R, k);
+    const bool in = !(past(p.x, R.dir.x, fx) || past(p.y, R.dir.y, fy) || past(p.z, R.dir.z, fz));
+    const bool out = past(q.x, R.dir.x, fx) || past(q.y, R.dir.y, fy) || past(q.z, R.dir.z, fz);
     const float n = k >= 1.0f && k < 1e29f && in && out ? k : k - 2.0f;
-    return fmaxf(fminf(n, ceilf(R.dist_e - R.dist_s)), 1.0f);
+    const float left = R.dist_e - R.dist_s;
+    return fmaxf(fminf(n, NEAR ? __fsub_rn(__fadd_ru(left, kFloorShift), kFloorShift) : ceilf(left)), 1.0f);
 }
 
 // The march loop, to a sample with sdf <= 0 or the end of the ray's range.
-template <int FMT>
+template <int FMT, bool NEAR>
 __device__ __forceinline__ void ray_march(const RayReader<FMT> &rd, float rstep, RayState &R) {
     int bx = INT_MIN, by = 0, bz = 0;  // the block of the sample at R.r
     int cptr = -1;                     // its pool index (-1: unallocated)
     bool jumped = false;               // the ray has taken its jump out of that (unallocated) block
     while (R.dist_s < R.dist_e) {
         float n = 1.0f;
-        const int vx = (int)floorf(R.r.x), vy = (int)floorf(R.r.y), vz = (int)floorf(R.r.z);
+        const int vx = ifloor_of<NEAR>(R.r.x), vy = ifloor_of<NEAR>(R.r.y), vz = ifloor_of<NEAR>(R.r.z);
         const int x = vx >> 3, y = vy >> 3, z = vz >> 3;
         if (x != bx || y != by || z != bz) {
             bx = x, by = y, bz = z;
@@ -399,24 +472,23 @@ __device__ __forceinline__ void ray_march(const RayReader<FMT> &rd, float rstep,
             cptr = rd.lookup(x, y, z);
         }
         if (cptr < 0) {
-            if (!jumped) n = empty_steps(R, (float)(vx & ~7), (float)(vy & ~7), (float)(vz & ~7));
+            if (!jumped) n = empty_steps<NEAR>(R, (float)(vx & ~7), (float)(vy & ~7), (float)(vz & ~7));
             jumped = true;
         } else {
             bool valid = true;
             R.sdf = rd.value(rd.at(cptr, vx, vy, vz), valid);
-            if (R.sdf <= 0.5f && R.sdf >= -0.5f) R.sdf = rd.interp(R.r, bx, by, bz, cptr, valid);
+            if (R.sdf <= 0.5f && R.sdf >= -0.5f) R.sdf = rd.template interp<NEAR>(R.r, bx, by, bz, cptr, valid);
             if (R.sdf <= 0.0f) return;
             if (valid) n = fmaxf(R.sdf * rstep, 1.0f);
         }
-        R.r.x += n * R.dir.x;
-        R.r.y += n * R.dir.y;
-        R.r.z += n * R.dir.z;
+        R.r = at_step(R, n);
         R.dist_s += n;
     }
 }
 
 // Vertex of a finished ray: a hit takes two interpolated correction steps
 // and is returned in camera coordinates (w = 1); a miss is NaN with w = -1.
+// (Its floors are the general ones: a stored sdf may move the ray anywhere.)
 template <int FMT>
 __device__ __forceinline__ float4 ray_finish(const RayReader<FMT> &rd, float rstep, float vsinv, const Rigid32 &Ti,
                                              RayState &R) {
@@ -430,7 +502,7 @@ __device__ __forceinline__ float4 ray_finish(const RayReader<FMT> &rd, float rst
         const int x = (int)floorf(R.r.x) >> 3, y = (int)floorf(R.r.y) >> 3, z = (int)floorf(R.r.z) >> 3;
         const int b = rd.lookup(x, y, z);
         bool valid = false;
-        R.sdf = b >= 0 ? rd.interp(R.r, x, y, z, b, valid) : 1.0f;
+        R.sdf = b >= 0 ? rd.template interp<false>(R.r, x, y, z, b, valid) : 1.0f;
         step = R.sdf * rstep;
         R.r.x += step * R.dir.x;
         R.r.y += step * R.dir.y;
@@ -449,10 +521,11 @@ __device__ __forceinline__ float4 ray_finish(const RayReader<FMT> &rd, float rst
 // is long when more than kLongBlocks blocks lie between the first visible
 // block in front of its pixels and the far bound of its tile.  Each tile is
 // launched for both turns, the long ones in the first half of the grid: a warp
-// of long rays takes most of the march's time wherever it starts (640x480, 5
-// mm: 97 us in image order, 85 with the long ones first; 4 or 32 blocks: 92
-// and 96).
-constexpr float kLongBlocks = 8.0f;
+// of long rays takes most of the march's time wherever it starts.  16 blocks:
+// with the raycast's other kernels, 106 us in a new map at 640x480, 5 mm and 219
+// in one of 1000 frames; 24 blocks: 108 and 220, 32: 113 and 240; 8: 240 in the
+// latter where 24 took 227.
+constexpr float kLongBlocks = 16.0f;
 template <int FMT>
 __device__ __forceinline__ void march_pixel(const MapDev &m, const Cam &cam, const PosePair *P,
                                             const float *__restrict__ znear, const float *__restrict__ zfar, int zw,
@@ -475,7 +548,11 @@ __device__ __forceinline__ void march_pixel(const MapDev &m, const Cam &cam, con
     }
     const bool live = inside && !skipped && ray_setup(cam, P->T, vsinv, zn, zf, zfine, x, y, R);
     const RayReader<FMT> rd(m, g);
-    if (live) ray_march(rd, rstep, R);
+    if (__all_sync(0xffffffffu, !live || ray_near(R))) {
+        if (live) ray_march<FMT, true>(rd, rstep, R);
+    } else {
+        if (live) ray_march<FMT, false>(rd, rstep, R);
+    }
     if (inside) vmap[(size_t)y * vpitch + x] = ray_finish(rd, rstep, vsinv, P->Tinv, R);
 }
 

@@ -187,7 +187,8 @@ struct VoxelIO<YAS_VOXEL_F16> {
     static constexpr int kBytes = 4;
     __device__ __forceinline__ static float sdf(T v) {
         const float h = __half2float(__ushort_as_half((unsigned short)(v & 0xffffu)));
-        const int q = (int)(v << 8) >> 24;
+        int q;  // byte 2, its sign copied into the bytes above
+        asm("prmt.b32 %0, %1, 0, 0xaaa2;" : "=r"(q) : "r"(v));
         return __int_as_float(__float_as_int(h) + q * 32);
     }
     __device__ __forceinline__ static int wt(T v) { return (int)(v >> 24); }
