@@ -552,7 +552,9 @@ class Canvas:
 
     def read(self):
         """(rgba (h, w, 4) uint8, depth (h, w) float32 metres, 0 where empty)."""
-        rgba = np.zeros((self.h, self.w, 4), np.uint8)
-        depth = np.zeros((self.h, self.w), np.float32)
+        rgba = np.empty((self.h, self.w, 4), np.uint8)
+        depth = np.empty((self.h, self.w), np.float32)
+        for a in (rgba, depth):  # every word is copied; a page new to the process is mapped sooner by the host
+            a.reshape(-1).view(np.uint8)[::4096] = 0
         L.call("yas_canvas_read", self.handle, rgba.ctypes.data, self.w * 4, depth.ctypes.data, self.w * 4, 0)
         return rgba, depth
