@@ -272,15 +272,13 @@ YAS_API int yas_map_fuse_depth(yas_map *m, const float *depth, int width, int he
                                      m->stream));
         d = (const float *)ex->depth.ptr;
     }
-    PosePair pp = make_pair(Tcm);
-    YAS_TRY_CUDA(cudaMemcpyAsync(m->pose_dev, &pp, sizeof(pp), cudaMemcpyHostToDevice, m->stream));
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, width, height);
     MapDev v = map_view(m);
     m->edits++;
-    launch_allocate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, nullptr, m->stream);
-    YAS_TRY_CUDA(cudaMemsetAsync(&m->hdr->n_visible, 0, sizeof(unsigned), m->stream));
-    launch_visible(v, cam, m->pose_dev, nullptr, m->stream);
-    launch_integrate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, nullptr, m->stream);
+    launch_pose_begin(v, make_pair(Tcm), m->pose_dev, m->stream);
+    launch_allocate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, nullptr, m->stream, true);
+    launch_visible(v, cam, m->pose_dev, nullptr, m->stream, true);
+    launch_integrate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, nullptr, m->stream, 0, true);
     YAS_TRY_CUDA(cudaGetLastError());
     if (!on_device) YAS_TRY_CUDA(cudaStreamSynchronize(m->stream));  // staging reuse safety
     return YAS_OK;
@@ -289,11 +287,9 @@ YAS_API int yas_map_fuse_depth(yas_map *m, const float *depth, int width, int he
 YAS_API int yas_map_check_visible(yas_map *m, int cols, int rows, const yas_pose *Tcm, unsigned *out) {
     if (!m || !Tcm || cols <= 0 || rows <= 0) return YAS_ERR_BAD_ARG;
     if (m->hibernated) return YAS_ERR_STATE;
-    PosePair pp = make_pair(Tcm);
-    YAS_TRY_CUDA(cudaMemcpyAsync(m->pose_dev, &pp, sizeof(pp), cudaMemcpyHostToDevice, m->stream));
-    YAS_TRY_CUDA(cudaMemsetAsync(&m->hdr->n_visible, 0, sizeof(unsigned), m->stream));
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, cols, rows);
-    launch_visible(map_view(m), cam, m->pose_dev, nullptr, m->stream);
+    launch_pose_begin(map_view(m), make_pair(Tcm), m->pose_dev, m->stream);
+    launch_visible(map_view(m), cam, m->pose_dev, nullptr, m->stream, true);
     YAS_TRY_CUDA(cudaGetLastError());
     if (out) {
         YAS_TRY(read_header(m));
@@ -869,13 +865,11 @@ YAS_API int yas_map_defuse_depth(yas_map *m, const float *depth, int width, int 
                                      m->stream));
         d = (const float *)ex->depth.ptr;
     }
-    PosePair pp = make_pair(Tcm);
-    YAS_TRY_CUDA(cudaMemcpyAsync(m->pose_dev, &pp, sizeof(pp), cudaMemcpyHostToDevice, m->stream));
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, width, height);
     MapDev v = map_view(m);
-    YAS_TRY_CUDA(cudaMemsetAsync(&m->hdr->n_visible, 0, sizeof(unsigned), m->stream));
-    launch_visible(v, cam, m->pose_dev, nullptr, m->stream);
-    launch_deintegrate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, m->stream);
+    launch_pose_begin(v, make_pair(Tcm), m->pose_dev, m->stream);
+    launch_visible(v, cam, m->pose_dev, nullptr, m->stream, true);
+    launch_deintegrate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, m->stream, true);
     YAS_TRY_CUDA(cudaGetLastError());
     if (!on_device) YAS_TRY_CUDA(cudaStreamSynchronize(m->stream));
     return YAS_OK;
@@ -895,7 +889,9 @@ YAS_API int yas_raycaster_create(yas_raycaster **out, int width, int height, con
     if (raycast_buffers_alloc(rc->rb, width, height) != YAS_OK ||
         cudaMalloc(&rc->vmap, (size_t)width * height * 16) != cudaSuccess ||
         cudaMalloc(&rc->depth_tmp, (size_t)width * height * 4) != cudaSuccess ||
-        cudaMalloc(&rc->pose_dev, sizeof(PosePair)) != cudaSuccess) {
+        cudaMalloc(&rc->pose_dev, sizeof(PosePair)) != cudaSuccess ||
+        cudaMallocHost(&rc->visible_host, sizeof(unsigned)) != cudaSuccess ||
+        cudaHostGetDevicePointer(reinterpret_cast<void **>(&rc->visible_dev), rc->visible_host, 0) != cudaSuccess) {
         cudaGetLastError();
         yas_raycaster_destroy(rc);
         return YAS_ERR_OOM;
@@ -918,6 +914,7 @@ YAS_API int yas_raycaster_destroy(yas_raycaster *rc) {
     cudaFree(rc->vmap);
     cudaFree(rc->depth_tmp);
     cudaFree(rc->pose_dev);
+    if (rc->visible_host) cudaFreeHost(rc->visible_host);
     delete rc;
     return YAS_OK;
 }
@@ -925,22 +922,15 @@ YAS_API int yas_raycaster_destroy(yas_raycaster *rc) {
 YAS_API int yas_raycaster_raycast(yas_raycaster *rc, yas_map *m, const yas_pose *Tcm) {
     if (!rc || !m || !Tcm) return YAS_ERR_BAD_ARG;
     if (m->hibernated) return YAS_ERR_STATE;
-    PosePair pp = make_pair(Tcm);
     cudaStream_t s = rc->stream;
     // The map's stream may differ: order the map's pending work first.
     if (m->stream != s) YAS_TRY_CUDA(cudaStreamSynchronize(m->stream));
-    YAS_TRY_CUDA(cudaMemcpyAsync(rc->pose_dev, &pp, sizeof(pp), cudaMemcpyHostToDevice, s));
-    YAS_TRY_CUDA(cudaMemsetAsync(&m->hdr->n_visible, 0, sizeof(unsigned), s));
-    MapDev v = map_view(m);
     Cam vis_cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, rc->w, rc->h);
-    launch_visible(v, vis_cam, rc->pose_dev, nullptr, s);
-    launch_zrange(v, rc->cam, rc->pose_dev, rc->rb, nullptr, s);
-    launch_march(v, m->cfg.voxel_format, rc->cam, rc->pose_dev, rc->rb, rc->vmap, rc->w, nullptr, s);
+    launch_raycast(map_view(m), m->cfg.voxel_format, vis_cam, rc->cam, make_pair(Tcm), rc->pose_dev, rc->rb, rc->vmap,
+                   rc->w, rc->visible_dev, s);
     YAS_TRY_CUDA(cudaGetLastError());
     YAS_TRY_CUDA(cudaStreamSynchronize(s));
-    MapHeader h;
-    YAS_TRY_CUDA(cudaMemcpy(&h, m->hdr, sizeof(h), cudaMemcpyDeviceToHost));
-    rc->last_visible = h.n_visible;
+    rc->last_visible = *static_cast<volatile unsigned *>(rc->visible_host);
     return YAS_OK;
 }
 
@@ -1131,8 +1121,13 @@ static int stage_input(yas_tracker *tr, const void *src, int pitch, int row_byte
         *dev_pitch = pitch;
         return YAS_OK;
     }
-    YAS_TRY_CUDA(cudaMemcpy2DAsync(tr->staging, row_bytes, src, pitch, row_bytes, tr->h, cudaMemcpyHostToDevice,
-                                   tr->stream));
+    // rows that adjoin are one copy: the row-wise one of pageable memory goes
+    // through the host (640x480: 48 us for an image or a depth, one copy 12 to 16)
+    if (pitch == row_bytes)
+        YAS_TRY_CUDA(cudaMemcpyAsync(tr->staging, src, (size_t)row_bytes * tr->h, cudaMemcpyHostToDevice, tr->stream));
+    else
+        YAS_TRY_CUDA(cudaMemcpy2DAsync(tr->staging, row_bytes, src, pitch, row_bytes, tr->h, cudaMemcpyHostToDevice,
+                                       tr->stream));
     *dev = tr->staging;
     *dev_pitch = row_bytes;
     return YAS_OK;

@@ -80,21 +80,18 @@ struct BlockLine {
 
 constexpr int kMaxLineBlocks = 1024;
 
-// Launches `k` on `s`; `dependent`: as a programmatic dependent of the
-// previous kernel on `s` (the kernel calls dependent_wait() first).
-template <typename... P, typename... A>
-static void launch_kernel(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, bool dependent, A... args) {
-    cudaLaunchConfig_t c = {};
-    c.gridDim = grid;
-    c.blockDim = block;
-    c.dynamicSmemBytes = 0;
-    c.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = at;
-    c.numAttrs = dependent ? 1 : 0;
-    cudaLaunchKernelEx(&c, k, args...);
+// Opens a call at a pose given by the host: one launch for a pose copy and a
+// memset, whose engine changes cost the call's chain twice as much.
+__global__ void pose_begin_kernel(PosePair pose, PosePair *P, MapHeader *hdr) {
+    release_dependents();
+    if (threadIdx.x == 0) {
+        *P = pose;
+        hdr->n_visible = 0u;
+    }
+}
+
+void launch_pose_begin(const MapDev &m, const PosePair &pose, PosePair *P, cudaStream_t s) {
+    pose_begin_kernel<<<1, 32, 0, s>>>(pose, P, m.hdr);
 }
 
 template <int VBYTES>
@@ -426,8 +423,8 @@ void launch_integrate(const MapDev &m, int fmt, const float *depth, int pitch_el
 }
 
 void launch_deintegrate(const MapDev &m, int fmt, const float *depth, int pitch_elems, const Cam &cam,
-                        const PosePair *P, cudaStream_t s) {
-    launch_integrate_sign<-1>(m, fmt, depth, pitch_elems, cam, P, nullptr, s);
+                        const PosePair *P, cudaStream_t s, bool dependent) {
+    launch_integrate_sign<-1>(m, fmt, depth, pitch_elems, cam, P, nullptr, s, 0, dependent);
 }
 
 // ---------------------------------------------------------------- reset

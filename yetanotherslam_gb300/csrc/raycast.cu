@@ -66,7 +66,7 @@ __device__ __forceinline__ bool grid_holds(int x, int y, int z) {
 
 // Opens an epoch: the grid is centred half way along the depth range, at most
 // 64 blocks ahead of the camera.  (grid_fill, the next kernel, writes info[4].)
-__device__ __forceinline__ void grid_begin(const MapDev &m, const PosePair *P, const BlockGrid &g) {
+__device__ __forceinline__ void grid_begin(const MapDev &m, const Rigid32 &T, const BlockGrid &g) {
     const int next = g.info[4], epoch = next < 1 || next > 255 ? 1 : next;
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     if (epoch == 1)
@@ -74,7 +74,7 @@ __device__ __forceinline__ void grid_begin(const MapDev &m, const PosePair *P, c
             reinterpret_cast<uint4 *>(g.cells)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (i0 == 0) {
         const float side = m.voxel_size * (float)kBlockSide;
-        const float3 c = rigid_fast(P->T, 0.0f, 0.0f, fminf(0.5f * m.depth_max, 64.0f * side));
+        const float3 c = rigid_fast(T, 0.0f, 0.0f, fminf(0.5f * m.depth_max, 64.0f * side));
         const float lim = 1.0e8f;  // far outside the key range
         g.info[0] = (int)floorf(fmaxf(-lim, fminf(lim, c.x / side))) - kGridSide / 2;
         g.info[1] = (int)floorf(fmaxf(-lim, fminf(lim, c.y / side))) - kGridSide / 2;
@@ -95,19 +95,35 @@ __device__ __forceinline__ void grid_fill(const MapDev &m, const BlockGrid &g) {
     if (blockIdx.x == 0 && threadIdx.x == 0) g.info[4] = g.info[3] + 1;
 }
 
-__global__ void zrange_reset_kernel(MapDev m, const PosePair *P, float *znear, float *zfar, int n, unsigned *queue,
-                                    float *fnear, int nf, BlockGrid g) {
+__device__ __forceinline__ void zrange_reset(const MapDev &m, const Rigid32 &T, float *znear, float *zfar, int n,
+                                             unsigned *queue, float *fnear, int nf, const BlockGrid &g) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         znear[i] = 100.0f;
         zfar[i] = 0.0f;
     }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nf; i += gridDim.x * blockDim.x) fnear[i] = 100.0f;
     if (blockIdx.x == 0 && threadIdx.x == 0) *queue = 0u;
-    grid_begin(m, P, g);
+    grid_begin(m, T, g);
+}
+
+__global__ void zrange_reset_kernel(MapDev m, const PosePair *P, float *znear, float *zfar, int n, unsigned *queue,
+                                    float *fnear, int nf, BlockGrid g) {
+    zrange_reset(m, P->T, znear, zfar, n, queue, fnear, nf, g);
+}
+
+// zrange_reset and pose_begin (map.cu) in one launch.
+__global__ void raycast_begin_kernel(MapDev m, PosePair pose, PosePair *P, float *znear, float *zfar, int n,
+                                     unsigned *queue, float *fnear, int nf, BlockGrid g) {
+    release_dependents();
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *P = pose;
+        m.hdr->n_visible = 0u;
+    }
+    zrange_reset(m, pose.T, znear, zfar, n, queue, fnear, nf, g);
 }
 
 __global__ void __launch_bounds__(256) grid_begin_kernel(MapDev m, const PosePair *P, BlockGrid g) {
-    grid_begin(m, P, g);
+    grid_begin(m, P->T, g);
 }
 
 __global__ void __launch_bounds__(256) grid_fill_kernel(MapDev m, BlockGrid g) {
@@ -134,10 +150,13 @@ __device__ __forceinline__ int clamp_ceil(float v) {
 __global__ void __launch_bounds__(128) zrange_fill_kernel(MapDev m, Cam cam, const PosePair *P,
                                                           float *znear, float *zfar, int zw, int zh,
                                                           const int *skip, float *fnear, int fw, int fh,
-                                                          BlockGrid g) {
+                                                          BlockGrid g, unsigned *host_visible) {
+    dependent_wait();
+    release_dependents();
     if (skip && *skip) return;
     grid_fill(m, g);
     const unsigned nvis = *(volatile unsigned *)&m.hdr->n_visible;
+    if (host_visible && blockIdx.x == 0 && threadIdx.x == 0) *host_visible = nvis;
     const Rigid32 Tinv = P->Tinv;
     const float scale = m.voxel_size * 8.0f;
     const unsigned lane = lane_id(), c = lane & 7u, shift = lane & ~7u;
@@ -233,7 +252,7 @@ void launch_zrange(const MapDev &m, const Cam &cam, const PosePair *P, RaycastBu
     zrange_reset_kernel<<<(std::max(n, nf) + 255) / 256, 256, 0, s>>>(m, P, rb.znear, rb.zfar, n, rb.queue, rb.fnear,
                                                                       nf, rb.grid);
     zrange_fill_kernel<<<kSMs * 8, 128, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, rb.zh, skip, rb.fnear, rb.fw,
-                                               rb.fh, rb.grid);
+                                               rb.fh, rb.grid, nullptr);
 }
 
 void launch_block_grid(const MapDev &m, const PosePair *P, const RaycastBuffers &rb, cudaStream_t s) {
@@ -567,6 +586,7 @@ __global__ void __launch_bounds__(32 * WX * WY) march_kernel(MapDev m, Cam cam, 
                                                              int vpitch, const int *skip,
                                                              const float *__restrict__ fnear, int fw, BlockGrid g) {
     constexpr int TX = RAYS == 32 ? 8 : 4, TY = RAYS / TX;
+    dependent_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int x = lane < RAYS ? (blockIdx.x * WX + warp % WX) * TX + lane % TX : INT_MAX;
     const int y = (blockIdx.y * WY + warp / WX) * TY + lane / TX;
@@ -648,12 +668,12 @@ static void launch_march_persistent(const MapDev &m, int fmt, const Cam &cam, co
 
 template <int WX, int WY, int RAYS>
 static void launch_march_rays(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, const RaycastBuffers &rb,
-                              float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s) {
+                              float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s, bool dependent) {
     constexpr int TX = (RAYS == 32 ? 8 : 4) * WX, TY = RAYS / (RAYS == 32 ? 8 : 4) * WY;
     const dim3 grid((cam.w + TX - 1) / TX, (cam.h + TY - 1) / TY, 2);
     const auto launch = [&](auto kernel) {
-        kernel<<<grid, 32 * WX * WY, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, vmap, vmap_pitch_elems, skip, rb.fnear,
-                                             rb.fw, rb.grid);
+        launch_kernel(kernel, grid, dim3(32 * WX * WY), s, dependent, m, cam, P, rb.znear, rb.zfar, rb.zw, vmap,
+                      vmap_pitch_elems, skip, rb.fnear, rb.fw, rb.grid);
     };
     switch (fmt) {
         case YAS_VOXEL_F32: launch(march_kernel<YAS_VOXEL_F32, WX, WY, RAYS>); break;
@@ -665,7 +685,8 @@ static void launch_march_rays(const MapDev &m, int fmt, const Cam &cam, const Po
 
 template <int WX, int WY>
 static void launch_march_tile(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, const RaycastBuffers &rb,
-                              float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s) {
+                              float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s,
+                              bool dependent = false) {
     // Rays per warp.  A small image does not fill the GPU with warps of 32 rays,
     // so a march lasts as long as its slowest warp, and that one ends sooner
     // with fewer rays: 320x240, 8 mm: 56 us at 32 rays, 50 at 16 and 49 at 8;
@@ -674,11 +695,11 @@ static void launch_march_tile(const MapDev &m, int fmt, const Cam &cam, const Po
     // 16, 149 at 8.
     const int px = cam.w * cam.h;
     if (px <= 40000)
-        launch_march_rays<WX, WY, 8>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s);
+        launch_march_rays<WX, WY, 8>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, dependent);
     else if (px <= 160000)
-        launch_march_rays<WX, WY, 16>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s);
+        launch_march_rays<WX, WY, 16>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, dependent);
     else
-        launch_march_rays<WX, WY, 32>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s);
+        launch_march_rays<WX, WY, 32>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, dependent);
 }
 
 void launch_march(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, const RaycastBuffers &rb,
@@ -689,6 +710,17 @@ void launch_march(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, c
         case 4: launch_march_tile<4, 1>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s); break;
         default: launch_march_tile<2, 2>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s); break;
     }
+}
+
+void launch_raycast(const MapDev &m, int fmt, const Cam &vis_cam, const Cam &cam, const PosePair &pose, PosePair *P,
+                    RaycastBuffers &rb, float4 *vmap, int vmap_pitch_elems, unsigned *host_visible, cudaStream_t s) {
+    const int n = rb.zw * rb.zh, nf = rb.fw * rb.fh;
+    raycast_begin_kernel<<<(std::max(n, nf) + 255) / 256, 256, 0, s>>>(m, pose, P, rb.znear, rb.zfar, n, rb.queue,
+                                                                       rb.fnear, nf, rb.grid);
+    launch_visible(m, vis_cam, P, nullptr, s, true);
+    launch_kernel(zrange_fill_kernel, dim3(kSMs * 8), dim3(128), s, true, m, cam, (const PosePair *)P, rb.znear, rb.zfar,
+                  rb.zw, rb.zh, (const int *)nullptr, rb.fnear, rb.fw, rb.fh, rb.grid, host_visible);
+    launch_march_tile<2, 2>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, nullptr, s, true);
 }
 
 __global__ void vmap_to_depth_kernel(const float4 *vmap, int vpitch, float *depth, int dpitch, int w,

@@ -65,7 +65,26 @@ int map_dev_alloc(yas_map *m);
 void map_dev_free(yas_map *m);
 MapDev map_view(const yas_map *m);
 
-// `dependent` (allocate, visible, integrate): launched as a programmatic
+// Launches `k` on `s`; `dependent`: as a programmatic dependent of the
+// previous kernel on `s` (the kernel calls dependent_wait() first).
+template <typename... P, typename... A>
+void launch_kernel(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, bool dependent, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = 0;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = dependent ? 1 : 0;
+    cudaLaunchKernelEx(&c, k, args...);
+}
+
+// The host's pose into *P, and an empty visible list.
+void launch_pose_begin(const MapDev &m, const PosePair &pose, PosePair *P, cudaStream_t s);
+// `dependent` (allocate, visible, integrate, march): launched as a programmatic
 // dependent of the previous kernel on `s`, which must be a kernel; its CTAs
 // are scheduled while that kernel finishes and wait for it in the kernel.
 // Allocates blocks along each depth ray (FP32-exact line tracing).
@@ -80,7 +99,7 @@ void launch_integrate(const MapDev &m, int fmt, const float *depth, int pitch_el
                       const PosePair *P, const int *skip, cudaStream_t s, int grid_ctas = 0,
                       bool dependent = false);
 void launch_deintegrate(const MapDev &m, int fmt, const float *depth, int pitch_elems, const Cam &cam,
-                        const PosePair *P, cudaStream_t s);
+                        const PosePair *P, cudaStream_t s, bool dependent = false);
 // Submap fusion and growth (fusion.cu)
 void launch_rehash(const MapDev &m, unsigned n, cudaStream_t s);
 void launch_fuse_alloc(const MapDev &dst, const MapDev &src, int fmt, const Rigid32 &T_src_dst, unsigned nsrc,
@@ -115,6 +134,12 @@ void raycast_buffers_free(RaycastBuffers &rb);
 // for a march at the same pose.
 void launch_zrange(const MapDev &m, const Cam &cam, const PosePair *P, RaycastBuffers &rb,
                    const int *skip, cudaStream_t s);
+// A raycast at a pose given by the host: the pose into *P, visibility (vis_cam),
+// z-range tiles, block grid and march, each a programmatic dependent of the one
+// before.  The length of the visible list also goes to *host_visible (mapped
+// host memory).
+void launch_raycast(const MapDev &m, int fmt, const Cam &vis_cam, const Cam &cam, const PosePair &pose, PosePair *P,
+                    RaycastBuffers &rb, float4 *vmap, int vmap_pitch_elems, unsigned *host_visible, cudaStream_t s);
 // The block grid alone, for a map whose blocks changed between launch_zrange
 // and the march.
 void launch_block_grid(const MapDev &m, const PosePair *P, const RaycastBuffers &rb, cudaStream_t s);
@@ -184,6 +209,8 @@ struct yas_raycaster {
     float *depth_tmp = nullptr;
     yas::PosePair *pose_dev = nullptr;
     unsigned last_visible = 0;
+    unsigned *visible_host = nullptr;  // mapped: the visible count of the last raycast
+    unsigned *visible_dev = nullptr;   // the same as the device maps it
 };
 
 struct yas_mesher {
