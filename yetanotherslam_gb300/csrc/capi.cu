@@ -114,6 +114,17 @@ using namespace yas;
 // Per-map staging for host depth in yas_map_fuse_depth.
 struct MapExtra {
     Staging depth;
+    cudaEvent_t copied = nullptr;  // the caller's depth has been read
+    ~MapExtra() {
+        if (copied) cudaEventDestroy(copied);
+    }
+    int take(const float *src, size_t bytes, cudaStream_t s) {
+        YAS_TRY(depth.ensure(bytes));
+        if (!copied) YAS_TRY_CUDA(cudaEventCreateWithFlags(&copied, cudaEventDisableTiming));
+        YAS_TRY_CUDA(cudaMemcpyAsync(depth.ptr, src, bytes, cudaMemcpyHostToDevice, s));
+        YAS_TRY_CUDA(cudaEventRecord(copied, s));
+        return YAS_OK;
+    }
 };
 static std::mutex g_extra_mutex;
 #include <unordered_map>
@@ -265,11 +276,9 @@ YAS_API int yas_map_fuse_depth(yas_map *m, const float *depth, int width, int he
         return YAS_ERR_BAD_ARG;
     if (m->hibernated) return YAS_ERR_STATE;
     const float *d = depth;
-    if (!on_device) {
-        MapExtra *ex = map_extra(m);
-        YAS_TRY(ex->depth.ensure((size_t)pitch_bytes * height));
-        YAS_TRY_CUDA(cudaMemcpyAsync(ex->depth.ptr, depth, (size_t)pitch_bytes * height, cudaMemcpyHostToDevice,
-                                     m->stream));
+    MapExtra *ex = on_device ? nullptr : map_extra(m);
+    if (ex) {
+        YAS_TRY(ex->take(depth, (size_t)pitch_bytes * height, m->stream));
         d = (const float *)ex->depth.ptr;
     }
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, width, height);
@@ -280,7 +289,8 @@ YAS_API int yas_map_fuse_depth(yas_map *m, const float *depth, int width, int he
     launch_visible(v, cam, m->pose_dev, nullptr, m->stream, true);
     launch_integrate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, nullptr, m->stream, 0, true);
     YAS_TRY_CUDA(cudaGetLastError());
-    if (!on_device) YAS_TRY_CUDA(cudaStreamSynchronize(m->stream));  // staging reuse safety
+    // the caller may write its depth again; the staging is reused in stream order
+    if (ex) YAS_TRY_CUDA(cudaEventSynchronize(ex->copied));
     return YAS_OK;
 }
 
@@ -858,11 +868,9 @@ YAS_API int yas_map_defuse_depth(yas_map *m, const float *depth, int width, int 
         return YAS_ERR_BAD_ARG;
     if (m->hibernated) return YAS_ERR_STATE;
     const float *d = depth;
-    if (!on_device) {
-        MapExtra *ex = map_extra(m);
-        YAS_TRY(ex->depth.ensure((size_t)pitch_bytes * height));
-        YAS_TRY_CUDA(cudaMemcpyAsync(ex->depth.ptr, depth, (size_t)pitch_bytes * height, cudaMemcpyHostToDevice,
-                                     m->stream));
+    MapExtra *ex = on_device ? nullptr : map_extra(m);
+    if (ex) {
+        YAS_TRY(ex->take(depth, (size_t)pitch_bytes * height, m->stream));
         d = (const float *)ex->depth.ptr;
     }
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, width, height);
@@ -871,7 +879,7 @@ YAS_API int yas_map_defuse_depth(yas_map *m, const float *depth, int width, int 
     launch_visible(v, cam, m->pose_dev, nullptr, m->stream, true);
     launch_deintegrate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, m->stream, true);
     YAS_TRY_CUDA(cudaGetLastError());
-    if (!on_device) YAS_TRY_CUDA(cudaStreamSynchronize(m->stream));
+    if (ex) YAS_TRY_CUDA(cudaEventSynchronize(ex->copied));
     return YAS_OK;
 }
 
