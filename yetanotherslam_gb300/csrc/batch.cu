@@ -215,6 +215,12 @@ static int plan_gn(yas_batch *b, const std::vector<uint8_t> &key, std::vector<GN
     return YAS_OK;
 }
 
+// Sessions from which on a step's raycasts fill the GPU beside one another
+// (steps of mixed sessions with the march's warps as for a shared GPU and as
+// for a lone one: one session 286 and 282 us, three 548 and 546, four 628 and
+// 638, eight 1251 and 1272).
+constexpr size_t kSharedSessions = 4;
+
 static int capture_step(yas_batch *b, const std::vector<uint8_t> &key, CachedStep &out) {
     std::vector<GNBatchItem> items;
     std::vector<unsigned short> cta_item;
@@ -269,7 +275,7 @@ static int capture_step(yas_batch *b, const std::vector<uint8_t> &key, CachedSte
         if (key[i] == kFirst) {
             session_enqueue_first(s);
         } else {
-            session_enqueue_pre(s);
+            session_enqueue_pre(s, items.size() >= kSharedSessions);
             if (chains) {  // the session's own GN launch, then its second half
                 const int k = item_of[i];
                 // the CTAs of one group fit the GPU together; a later group's

@@ -686,29 +686,29 @@ static void launch_march_rays(const MapDev &m, int fmt, const Cam &cam, const Po
 template <int WX, int WY>
 static void launch_march_tile(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, const RaycastBuffers &rb,
                               float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s,
-                              bool dependent = false) {
+                              bool dependent = false, bool shared = false) {
     // Rays per warp.  A small image does not fill the GPU with warps of 32 rays,
     // so a march lasts as long as its slowest warp, and that one ends sooner
     // with fewer rays: 320x240, 8 mm: 56 us at 32 rays, 50 at 16 and 49 at 8;
     // 160x120, 1 cm: 51 at 32 and 38 at 8.  In larger images instruction issue
     // counts, and full warps take the fewest: 640x480, 5 mm: 79 us at 32, 96 at
-    // 16, 149 at 8.
+    // 16, 149 at 8.  So they do where the marches of several sessions fill the GPU.
     const int px = cam.w * cam.h;
-    if (px <= 40000)
+    if (px <= 40000 && !shared)
         launch_march_rays<WX, WY, 8>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, dependent);
-    else if (px <= 160000)
+    else if (px <= 160000 && !shared)
         launch_march_rays<WX, WY, 16>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, dependent);
     else
         launch_march_rays<WX, WY, 32>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, dependent);
 }
 
 void launch_march(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, const RaycastBuffers &rb,
-                  float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s, int tile) {
+                  float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s, int tile, bool shared) {
     switch (tile) {
         case 0: launch_march_persistent(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s); break;
-        case 1: launch_march_tile<1, 4>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s); break;
-        case 4: launch_march_tile<4, 1>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s); break;
-        default: launch_march_tile<2, 2>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s); break;
+        case 1: launch_march_tile<1, 4>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, false, shared); break;
+        case 4: launch_march_tile<4, 1>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, false, shared); break;
+        default: launch_march_tile<2, 2>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, false, shared); break;
     }
 }
 

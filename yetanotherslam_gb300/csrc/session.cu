@@ -276,12 +276,12 @@ static void enqueue_first_frame(yas_session *s) {
 // (Tracking.cpp:164-169): reads the map, the pose pair and the z-range tiles
 // the previous frame's fusion left, writes the reference set's vertex/normal
 // maps only.
-static void enqueue_raycast_branch(yas_session *s, cudaStream_t st) {
+static void enqueue_raycast_branch(yas_session *s, cudaStream_t st, bool shared) {
     yas_tracker *tr = s->tr;
     MapDev v = map_view(s->map);
     prof_mark(s, kStMarch);
     launch_march(v, s->map->cfg.voxel_format, s->rc->cam, &s->fs->pp, s->zt, tr->refb(0).vmap, s->cfg.width,
-                 nullptr, st, s->shape.march_warps_x);
+                 nullptr, st, s->shape.march_warps_x, shared);
     prof_mark(s, kStModel);
     tracker_model(tr, st);
 }
@@ -300,8 +300,9 @@ static void enqueue_frame_branch(yas_session *s, cudaStream_t st) {
 }
 
 // A tracked frame up to the Gauss-Newton schedule: pyramids of the new frame,
-// raycast of the map and model pyramid, GN state reset.
-static void enqueue_pre(yas_session *s) {
+// raycast of the map and model pyramid, GN state reset.  `shared`: beside those
+// of several other sessions (launch_march).
+static void enqueue_pre_as(yas_session *s, bool shared) {
     yas_tracker *tr = s->tr;
     cudaStream_t st = s->stream;
     if (s->side && !s->profiling) {
@@ -310,18 +311,20 @@ static void enqueue_pre(yas_session *s) {
         // frame branch, off the raycast's path
         cudaEventRecord(s->ev_fork, st);
         cudaStreamWaitEvent(s->side, s->ev_fork, 0);
-        enqueue_raycast_branch(s, s->side);
+        enqueue_raycast_branch(s, s->side, shared);
         enqueue_frame_branch(s, st);
         launch_gn_init(tr, pose_identity(), st);
         cudaEventRecord(s->ev_join, s->side);
         cudaStreamWaitEvent(st, s->ev_join, 0);
     } else {
         enqueue_frame_branch(s, st);
-        enqueue_raycast_branch(s, st);
+        enqueue_raycast_branch(s, st, shared);
         prof_mark(s, kStGnInit);
         launch_gn_init(tr, pose_identity(), st);
     }
 }
+
+static void enqueue_pre(yas_session *s) { enqueue_pre_as(s, false); }
 
 // A tracked frame after the Gauss-Newton schedule: pose update (its result
 // written to the host's copy too), fusion.  `dependent`: the fusion kernels
@@ -566,7 +569,7 @@ void session_set_shape(yas_session *s, const LaunchShape &shape) {
 const LaunchShape &session_shape(const yas_session *s) { return s->shape; }
 
 void session_enqueue_first(yas_session *s) { enqueue_first_frame(s); }
-void session_enqueue_pre(yas_session *s) { enqueue_pre(s); }
+void session_enqueue_pre(yas_session *s, bool shared) { enqueue_pre_as(s, shared); }
 void session_enqueue_post(yas_session *s) { enqueue_post(s); }
 
 void session_finish_first(yas_session *s) { s->frames++; }

@@ -146,9 +146,11 @@ void launch_block_grid(const MapDev &m, const PosePair *P, const RaycastBuffers 
 // `warps_x` 1, 2 (the default), 4: one thread per pixel, a 128-thread CTA's
 // four 8x4-pixel warp tiles side by side in x (8x16, 16x8, 32x4 pixels);
 // 0: persistent warps taking 8x4-pixel tiles from a queue.  The output is
-// the same.
+// the same.  `shared`: several marches run beside one another, so warps take 32
+// rays whatever the image.
 void launch_march(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, const RaycastBuffers &rb,
-                  float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s, int warps_x = 2);
+                  float4 *vmap, int vmap_pitch_elems, const int *skip, cudaStream_t s, int warps_x = 2,
+                  bool shared = false);
 void launch_vmap_to_depth(const float4 *vmap, int vpitch, float *depth, int dpitch, int w, int h,
                           cudaStream_t s);
 

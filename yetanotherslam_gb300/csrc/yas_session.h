@@ -43,7 +43,7 @@ const LaunchShape &session_shape(const yas_session *s);
 // that captures many sessions into one graph (the batch): the initialising
 // frame, or a tracked frame's halves around the Gauss-Newton schedule.
 void session_enqueue_first(yas_session *s);
-void session_enqueue_pre(yas_session *s);
+void session_enqueue_pre(yas_session *s, bool shared);
 void session_enqueue_post(yas_session *s);
 // Bookkeeping after such a frame has been launched.
 void session_finish_first(yas_session *s);
