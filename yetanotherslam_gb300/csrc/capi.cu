@@ -88,6 +88,39 @@ static PosePair make_pair(const yas_pose *Tcm) {
 
 static bool is_pow2(long long v) { return v > 0 && (v & (v - 1)) == 0; }
 
+// Sixteen bytes a thread; one more thread takes the bytes that are left.
+__global__ void __launch_bounds__(256) read_in_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst,
+                                                      size_t bytes) {
+    const size_t at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 16;
+    if (at + 16 <= bytes)
+        *reinterpret_cast<uint4 *>(dst + at) = *reinterpret_cast<const uint4 *>(src + at);
+    else
+        for (size_t i = at; i < bytes; ++i) dst[i] = src[i];
+}
+
+// A host input into device memory; the caller waits before it gives the input
+// back.  A copy of pageable memory holds the host until it is done (11 us for
+// 300 KB, 17 for 1.2 MB, at 190 GB/s when it runs); where the device reads such
+// memory through the process's page tables, a kernel does, and the launches
+// that follow it are enqueued meanwhile.
+int copy_in(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+    if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0 && bytes < (1ull << 40)) {
+        int dev = 0, pageable = 0;
+        cudaPointerAttributes a;
+        if (cudaGetDevice(&dev) == cudaSuccess &&
+            cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess && pageable &&
+            cudaPointerGetAttributes(&a, src) == cudaSuccess && a.type == cudaMemoryTypeUnregistered) {
+            read_in_kernel<<<(unsigned)((bytes + 4095) / 4096), 256, 0, s>>>(static_cast<const uint8_t *>(src),
+                                                                            static_cast<uint8_t *>(dst), bytes);
+            YAS_TRY_CUDA(cudaGetLastError());
+            return YAS_OK;
+        }
+        cudaGetLastError();
+    }
+    YAS_TRY_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+    return YAS_OK;
+}
+
 // Device staging buffer for host inputs, grown on demand.
 struct Staging {
     void *ptr = nullptr;
@@ -121,7 +154,7 @@ struct MapExtra {
     int take(const float *src, size_t bytes, cudaStream_t s) {
         YAS_TRY(depth.ensure(bytes));
         if (!copied) YAS_TRY_CUDA(cudaEventCreateWithFlags(&copied, cudaEventDisableTiming));
-        YAS_TRY_CUDA(cudaMemcpyAsync(depth.ptr, src, bytes, cudaMemcpyHostToDevice, s));
+        YAS_TRY(copy_in(depth.ptr, src, bytes, s));
         YAS_TRY_CUDA(cudaEventRecord(copied, s));
         return YAS_OK;
     }
@@ -1132,7 +1165,7 @@ static int stage_input(yas_tracker *tr, const void *src, int pitch, int row_byte
     // rows that adjoin are one copy: the row-wise one of pageable memory goes
     // through the host (640x480: 48 us for an image or a depth, one copy 12 to 16)
     if (pitch == row_bytes)
-        YAS_TRY_CUDA(cudaMemcpyAsync(tr->staging, src, (size_t)row_bytes * tr->h, cudaMemcpyHostToDevice, tr->stream));
+        YAS_TRY(copy_in(tr->staging, src, (size_t)row_bytes * tr->h, tr->stream));
     else
         YAS_TRY_CUDA(cudaMemcpy2DAsync(tr->staging, row_bytes, src, pitch, row_bytes, tr->h, cudaMemcpyHostToDevice,
                                        tr->stream));

@@ -190,6 +190,7 @@ struct yas_session {
     const void *input_src[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // the nodes' current sources
     bool capture_input = false;  // capturing exec[]: the frame branch starts with the input copy
     int device = 0;
+    bool reads_pageable = false;  // the device reads pageable host memory in place
     cudaGraphExec_t pre_exec[2] = {nullptr, nullptr};  // served frames: up to the GN schedule
     cudaGraphExec_t post_exec = nullptr;               // served frames: after it
     // the map's device arrays when the graphs were captured: growth, fusion
@@ -422,8 +423,11 @@ static void launch_input_copy(yas_session *s, cudaStream_t st) {
 }
 
 // Device address of `bytes` of a frame input the input copy kernel can read:
-// 16-byte aligned memory of this device (on_device) or pinned host memory the
-// device maps; null otherwise (the copy then runs on the stream).
+// 16-byte aligned memory of this device (on_device), or host memory that the
+// device maps (pinned) or reaches through the process's own page tables (any);
+// null otherwise (the copy then runs on the stream, and one of pageable memory
+// holds the host until it is done: two of them before every frame's launch, 20
+// us of a 320x240 frame).
 static const void *readable_input(const yas_session *s, const void *p, size_t bytes, int on_device) {
     if ((reinterpret_cast<uintptr_t>(p) & 15u) || (bytes & 15u)) return nullptr;
     cudaPointerAttributes a;
@@ -431,9 +435,9 @@ static const void *readable_input(const yas_session *s, const void *p, size_t by
         cudaGetLastError();
         return nullptr;
     }
-    const bool ok = on_device ? (a.type == cudaMemoryTypeDevice && a.device == s->device)
-                              : a.type == cudaMemoryTypeHost;
-    return ok ? a.devicePointer : nullptr;
+    if (on_device) return a.type == cudaMemoryTypeDevice && a.device == s->device ? a.devicePointer : nullptr;
+    if (a.type == cudaMemoryTypeUnregistered) return s->reads_pageable ? p : nullptr;
+    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
 // Points the input copy node of exec[parity] at this frame's sources (null:
@@ -628,6 +632,9 @@ YAS_API int yas_session_create(yas_session **out, const yas_session_config *cfg,
         delete s;
         return YAS_ERR_CUDA;
     }
+    int pageable = 0;
+    if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, s->device) != cudaSuccess) cudaGetLastError();
+    s->reads_pageable = pageable != 0;
     if (stream) {
         s->stream = (cudaStream_t)stream;
     } else {
