@@ -81,7 +81,8 @@ struct BlockLine {
 constexpr int kMaxLineBlocks = 1024;
 
 // Opens a call at a pose given by the host: one launch for a pose copy and a
-// memset, whose engine changes cost the call's chain twice as much.
+// memset.  With the call's kernels as dependents, one Fuse after another 160x120
+// 23.1 / 16.9 us, 640x480 43.0 / 36.0.
 __global__ void pose_begin_kernel(PosePair pose, PosePair *P, MapHeader *hdr) {
     release_dependents();
     if (threadIdx.x == 0) {
