@@ -1222,9 +1222,12 @@ YAS_API int yas_tracker_get_transform(yas_tracker *tr, const yas_pose *init, int
     if (!tr || !out) return YAS_ERR_BAD_ARG;
     Pose64 p0 = init ? pose_from(*init) : pose_identity();
     launch_gn_init(tr, p0, tr->stream);
-    launch_gn_schedule(tr, tr->stream);
+    // the schedule writes its result here, unless one of its waits gives up
+    tr->state_host->failed = kFailTimeout;
+    const bool written = launch_gn_schedule(tr, tr->stream, tr->state_host_dev);
     YAS_TRY_CUDA(cudaGetLastError());
-    YAS_TRY_CUDA(cudaMemcpyAsync(tr->state_host, tr->state, sizeof(GNState), cudaMemcpyDeviceToHost, tr->stream));
+    if (!written)
+        YAS_TRY_CUDA(cudaMemcpyAsync(tr->state_host, tr->state, sizeof(GNState), cudaMemcpyDeviceToHost, tr->stream));
     YAS_TRY_CUDA(cudaStreamSynchronize(tr->stream));
     const GNState &st = *tr->state_host;
     if (st.failed) {

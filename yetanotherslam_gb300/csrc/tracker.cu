@@ -581,6 +581,7 @@ struct FusedArgs {
     unsigned long long *rows;  // [2 parities][2 passes][kFusedMaxCtas][32] tagged words
     float4 *res4;              // per-pixel residuals of the PIX == 0 schedule (level-0 sized)
     GNState *st;
+    GNState *host;             // mapped host memory for the result (null: none)
 };
 
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
@@ -967,7 +968,7 @@ __device__ __forceinline__ bool fold_systems(const unsigned long long *rowsA, co
 template <int PIX, int NT, int MODE>
 __device__ __forceinline__ void gn_schedule(const FusedLevel *lvs, int L, int mode_, IcpGates gates,
                                             unsigned long long *rows, float4 *res4, GNState *st, unsigned cta,
-                                            unsigned nrows) {
+                                            unsigned nrows, GNState *host) {
     __shared__ float sRK[9];
     const int t = (int)threadIdx.x;
     const int mode = MODE != 0 ? MODE : mode_;
@@ -1107,13 +1108,18 @@ __device__ __forceinline__ void gn_schedule(const FusedLevel *lvs, int L, int mo
         publish_solve(st);
         st->a_sums[t] = df_to_double(total(0, t));
         st->b_sums[t] = df_to_double(total(1, t));
+        if (host) {
+            if (t < 12) host->best[t] = df_to_double(DF{g_solve.besth[t], g_solve.bestl[t]});
+            if (t == 12) host->failed = g_solve.failed;
+        }
     }
 }
 
 // The fused schedule of one tracker over the whole grid.
 template <int PIX, int MODE>
 __global__ void __launch_bounds__(fused_threads<PIX>(), 1) gn_fused(const __grid_constant__ FusedArgs a) {
-    gn_schedule<PIX, fused_threads<PIX>(), MODE>(a.lv, a.L, a.mode, a.gates, a.rows, a.res4, a.st, blockIdx.x, gridDim.x);
+    gn_schedule<PIX, fused_threads<PIX>(), MODE>(a.lv, a.L, a.mode, a.gates, a.rows, a.res4, a.st, blockIdx.x, gridDim.x,
+                                                a.host);
 }
 
 // Fused schedules of a batch of trackers in one launch: CTA b runs for item
@@ -1127,7 +1133,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) gn_fused_batch(const GNBatch
                                                                     const unsigned short *__restrict__ cta_item) {
     const GNBatchItem &it = items[cta_item[blockIdx.x]];
     gn_schedule<PIX, kBatchThreads, MODE>(it.lv, it.L, it.mode, it.gates, it.rows, it.res4, it.st,
-                                    blockIdx.x - (unsigned)it.cta0, (unsigned)it.nctas);
+                                    blockIdx.x - (unsigned)it.cta0, (unsigned)it.nctas, nullptr);
 }
 
 // ---------------------------------------------------------------- host side
@@ -1305,7 +1311,7 @@ static void fill_levels(yas_tracker *tr, int grid, int threads, FusedLevel *lv) 
     }
 }
 
-static bool launch_gn_fused(yas_tracker *tr, cudaStream_t s) {
+static bool launch_gn_fused(yas_tracker *tr, cudaStream_t s, GNState *host) {
     int pix = 0, grid = 0;
     if (!tr->use_fused || !fused_plan(tr, pix, grid)) return false;
     FusedArgs a;
@@ -1317,6 +1323,7 @@ static bool launch_gn_fused(yas_tracker *tr, cudaStream_t s) {
     a.rows = tr->fused_rows;
     a.res4 = tr->res4;
     a.st = tr->state;
+    a.host = host;
     if (tr->hook) tr->hook(tr->hook_ctx, 30);
     const cudaError_t e = pix == 1   ? launch_fused_pix<1>(a, grid, s)
                           : pix == 2 ? launch_fused_pix<2>(a, grid, s)
@@ -1412,10 +1419,11 @@ cudaError_t launch_gn_batch(const GNBatchItem *dev_items, const unsigned short *
     }
 }
 
-void launch_gn_schedule(yas_tracker *tr, cudaStream_t s) {
-    if (launch_gn_fused(tr, s)) return;
+bool launch_gn_schedule(yas_tracker *tr, cudaStream_t s, GNState *host) {
+    if (launch_gn_fused(tr, s, host)) return host != nullptr;
     for (int l = tr->L - 1; l >= 0; --l)
         for (int it = 0; it < tr->iters[l]; ++it) launch_gn_iteration(tr, l, it == 0, s);
+    return false;
 }
 
 void launch_gn_linearise(yas_tracker *tr, int l, cudaStream_t s) { launch_passes(tr, l, 0, 1, s); }
@@ -1458,7 +1466,8 @@ int tracker_alloc(yas_tracker *tr) {
     tr->staging = grab(tr->staging_bytes);
     if (!tr->res4 || !tr->partialA || !tr->partialB || !tr->growA || !tr->growB || !tr->counters || !tr->fused_rows || !tr->state || !tr->staging)
         return YAS_ERR_OOM;
-    if (cudaMallocHost(&tr->state_host, sizeof(GNState)) != cudaSuccess) {
+    if (cudaMallocHost(&tr->state_host, sizeof(GNState)) != cudaSuccess ||
+        cudaHostGetDevicePointer(reinterpret_cast<void **>(&tr->state_host_dev), tr->state_host, 0) != cudaSuccess) {
         cudaGetLastError();
         return YAS_ERR_OOM;
     }

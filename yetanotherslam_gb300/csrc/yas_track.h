@@ -124,6 +124,7 @@ struct yas_tracker {
     int fused_max_grid[4] = {-1, -1, -1, -1};  // co-resident CTAs for 1, 2, 4 pixels per thread, and any
     yas::GNState *state = nullptr;
     yas::GNState *state_host = nullptr;  // pinned
+    yas::GNState *state_host_dev = nullptr;  // the same as the device maps it
     void *staging = nullptr;             // host-input staging (w*h*4 bytes)
     size_t staging_bytes = 0;
     bool good = true;
@@ -147,7 +148,9 @@ void launch_gn_init(yas_tracker *tr, const Pose64 &init, cudaStream_t s);
 // One GN iteration at level l (pass A, and pass B for modes with RGB).
 void launch_gn_iteration(yas_tracker *tr, int l, bool first_of_level, cudaStream_t s);
 // Full coarse-to-fine schedule (GetTransform without the swap).
-void launch_gn_schedule(yas_tracker *tr, cudaStream_t s);
+// `host`: where the fused schedule also writes the kept estimate and whether it
+// failed (mapped memory; left as it is when a wait gives up); true if it does.
+bool launch_gn_schedule(yas_tracker *tr, cudaStream_t s, GNState *host = nullptr);
 // Preprocessing of current / reference frames from device sources.
 void tracker_image(yas_tracker *tr, const uint8_t *src, int channels, int pitch, bool reference,
                    cudaStream_t s);
