@@ -108,7 +108,8 @@ int copy_in(void *dst, const void *src, size_t bytes, cudaStream_t s) {
         int dev = 0, pageable = 0;
         cudaPointerAttributes a;
         if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess && pageable &&
+            cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) == cudaSuccess &&
+            pageable &&
             cudaPointerGetAttributes(&a, src) == cudaSuccess && a.type == cudaMemoryTypeUnregistered) {
             read_in_kernel<<<(unsigned)((bytes + 4095) / 4096), 256, 0, s>>>(static_cast<const uint8_t *>(src),
                                                                             static_cast<uint8_t *>(dst), bytes);

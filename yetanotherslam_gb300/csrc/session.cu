@@ -633,7 +633,8 @@ YAS_API int yas_session_create(yas_session **out, const yas_session_config *cfg,
         return YAS_ERR_CUDA;
     }
     int pageable = 0;
-    if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, s->device) != cudaSuccess) cudaGetLastError();
+    if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccessUsesHostPageTables, s->device) != cudaSuccess)
+        cudaGetLastError();
     s->reads_pageable = pageable != 0;
     if (stream) {
         s->stream = (cudaStream_t)stream;
