@@ -450,6 +450,9 @@ class Session:
         lib = L.load()
         self._submit_fn, self._wait_fn = lib.yas_session_submit, lib.yas_session_wait
         self._pose, self._status = L.Pose(), C.c_int()
+        # inputs of the frames submitted since the last wait: the GPU reads them
+        # in place, and several frames may be in flight
+        self._keep = []
 
     def close(self):
         if self.handle:
@@ -467,11 +470,12 @@ class Session:
         dp, _, ddev, k2 = _device_info(depth)
         if rdev != ddev:
             raise ValueError("rgb and depth must both be host or both be device arrays")
-        self._keep = (k1, k2)
+        self._keep.append((k1, k2))
         L.check(self._submit_fn(self.handle, rp, dp, rdev), "yas_session_submit")
 
     def wait(self):
         L.check(self._wait_fn(self.handle, C.byref(self._pose), C.byref(self._status)), "yas_session_wait")
+        self._keep.clear()
         return self._status.value, L.pose_to(self._pose)
 
     def process(self, rgb, depth):
