@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstring>
 
+#include "pure.h"
 #include "yas_track.h"
 
 namespace yas {
@@ -312,7 +313,7 @@ YAS_API int yas_map_fuse_depth(yas_map *m, const float *depth, int width, int he
     const float *d = depth;
     MapExtra *ex = on_device ? nullptr : map_extra(m);
     if (ex) {
-        YAS_TRY(ex->take(depth, (size_t)pitch_bytes * height, m->stream));
+        YAS_TRY(ex->take(depth, image_bytes((size_t)width * 4, (size_t)pitch_bytes, height), m->stream));
         d = (const float *)ex->depth.ptr;
     }
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, width, height);
@@ -904,7 +905,7 @@ YAS_API int yas_map_defuse_depth(yas_map *m, const float *depth, int width, int 
     const float *d = depth;
     MapExtra *ex = on_device ? nullptr : map_extra(m);
     if (ex) {
-        YAS_TRY(ex->take(depth, (size_t)pitch_bytes * height, m->stream));
+        YAS_TRY(ex->take(depth, image_bytes((size_t)width * 4, (size_t)pitch_bytes, height), m->stream));
         d = (const float *)ex->depth.ptr;
     }
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, width, height);
