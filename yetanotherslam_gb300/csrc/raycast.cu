@@ -40,6 +40,7 @@
 #include <cfloat>
 #include <climits>
 
+#include "pure.h"
 #include "yas_internal.h"
 
 namespace yas {
@@ -57,7 +58,6 @@ namespace yas {
 // the grid, and those whose index does not fit 24 bits (kGridAsk), are looked
 // up in the table.
 // info: first block x, y, z; epoch; epoch of the next raycast.
-constexpr unsigned kGridAsk = 0xffffffu;
 
 __device__ __forceinline__ int grid_cell(int x, int y, int z) { return (z * kGridSide + y) * kGridSide + x; }
 __device__ __forceinline__ bool grid_holds(int x, int y, int z) {
@@ -339,29 +339,13 @@ struct RayReader {
         for (int c = 0; c < 8; ++c) q[c] = (unsigned)b;
         if (across != 0u) {
             const int gx = bx - ox, gy = by - oy, gz = bz - oz;
-            bool ask = true;
-            lim = kGridAsk;
-            if (max(max((unsigned)gx, (unsigned)gy), (unsigned)gz) < (unsigned)(kGridSide - 1)) {
-                const unsigned *cell = g.cells + grid_cell(gx, gy, gz);
-                const int sx = across & 1u, sy = across & 2u ? kGridSide : 0, sz = across & 4u ? kGridSide * kGridSide : 0;
-                ask = false;
-#pragma unroll
-                for (int c = 1; c < 8; ++c) {
-                    q[c] = __ldg(cell + ((c & 1 ? sx : 0) + (c & 2 ? sy : 0) + (c & 4 ? sz : 0))) - epoch;
-                    ask = ask || q[c] == kGridAsk;
-                }
-            }
-            if (ask) {
-                lim = 0x80000000u;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) q[c] = (unsigned)b;
-#pragma unroll 1
-                for (unsigned d = across; d != 0u; d = (d - 1u) & across) {
-                    const int e = lookup(bx + (int)(d & 1u), by + (int)((d >> 1) & 1u), bz + (int)(d >> 2));
-#pragma unroll
-                    for (unsigned c = 1u; c < 8u; ++c) q[c] = (c & across) == d ? (unsigned)e : q[c];
-                }
-            }
+            const bool inner = max(max((unsigned)gx, (unsigned)gy), (unsigned)gz) < (unsigned)(kGridSide - 1);
+            const unsigned *cell = g.cells + (inner ? grid_cell(gx, gy, gz) : 0);
+            const int sx = across & 1u, sy = across & 2u ? kGridSide : 0, sz = across & 4u ? kGridSide * kGridSide : 0;
+            lim = corner_blocks(
+                across, b, inner,
+                [&](unsigned c) { return __ldg(cell + ((c & 1 ? sx : 0) + (c & 2 ? sy : 0) + (c & 4 ? sz : 0))) - epoch; },
+                [&](unsigned d) { return lookup(bx + (int)(d & 1u), by + (int)((d >> 1) & 1u), bz + (int)(d >> 2)); }, q);
         }
         const int xo[2] = {x0 & 7, (x0 + 1) & 7}, yo[2] = {(y0 & 7) << 3, ((y0 + 1) & 7) << 3};
         const int zo[2] = {(z0 & 7) << 6, ((z0 + 1) & 7) << 6};
