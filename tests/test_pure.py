@@ -43,6 +43,9 @@ extern "C" int corner_mismatches(int cells, int inner) {
 }
 
 extern "C" size_t image_bytes(size_t row, size_t pitch, int rows) { return yas::image_bytes(row, pitch, rows); }
+extern "C" void huber_scaled(const float *sd, float *out, int n) {
+    for (int i = 0; i < n; ++i) out[i] = yas::huber_scaled(sd[i]);
+}
 """
 
 
@@ -68,3 +71,14 @@ def test_an_image_ends_with_its_last_rows_own_bytes(pure, w, h, pad):
 @pytest.mark.parametrize("inner", [0, 1])
 def test_corner_blocks_at_the_grids_index_limit(pure, inner):
     assert pure.corner_mismatches(200000, inner) == 0
+
+
+def test_huber_scale_rounds_once(pure):
+    """Every deviation of two binades, and the ends of the range."""
+    sd = np.concatenate([np.arange(0x3f800000, 0x40800000, dtype=np.uint32).view(np.float32),
+                         np.array([0, 1e-45, 1e-38, 7e37, 3.4e38, np.inf, np.nan], np.float32)])
+    out = np.empty_like(sd)
+    pure.huber_scaled(sd.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p), sd.size)
+    with np.errstate(over="ignore"):
+        want = (4.685 * sd.astype(np.float64)).astype(np.float32)
+    assert np.array_equal(out.view(np.uint32)[:-1], want.view(np.uint32)[:-1]) and np.isnan(out[-1])

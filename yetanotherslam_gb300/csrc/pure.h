@@ -21,6 +21,11 @@ namespace yas {
 // image's, and need not be there.
 inline size_t image_bytes(size_t row_bytes, size_t pitch, int rows) { return pitch * (size_t)(rows - 1) + row_bytes; }
 
+// 4.685 sd, the FP64 product rounded once to FP32.  (An FP32 product with 4.685 to
+// 48 bits, its parts summed, is a last place off for one sd in 2800, on the wrong
+// side of a near tie, and is not a number for an infinite one.)
+YAS_PURE float huber_scaled(float sd) { return (float)(4.685 * (double)sd); }
+
 // A cell of a raycast's block grid, its epoch taken off: a pool index below
 // kGridAsk; kGridAsk where the index does not fit (the hash table has it); above,
 // no allocated block.

@@ -38,6 +38,7 @@
 #include <cuda.h>
 
 #include "gn_solve.cuh"
+#include "pure.h"
 #include "yas_track.h"
 
 namespace yas {
@@ -385,11 +386,7 @@ __device__ __forceinline__ float huber_threshold_df(DF nn, DF s, DF s2) {
     const DF md = df(mean);
     const DF ss = df_fma(df_mul(nn, md), md, df_fma(df(-2.0f * mean), s, s2));
     const float var = sqrtf(ss.h / (nn.h - 1.0f));
-    // 4.685 var from its product with 4.685 to 48 bits, rounded once (an FP64
-    // product costs three serial FP64 instructions of some 65 cycles each)
-    constexpr float ch = 4.685f, cl = (float)(4.685 - (double)ch);
-    const float p = __fmul_rn(ch, var);
-    return __fadd_rn(p, __fmaf_rn(cl, var, __fmaf_rn(ch, var, -p)));
+    return huber_scaled(var);
 }
 __device__ __forceinline__ float huber_threshold(const double *tot) {
     return huber_threshold_df(df_from_double(tot[29]), df_from_double(tot[30]), df_from_double(tot[31]));
