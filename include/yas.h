@@ -112,7 +112,9 @@ YAS_API int yas_map_reset(yas_map *map);
 /* MapStruct::Empty(): VoxelMap.h:46 / VoxelMap.cu:138-141 (no allocated block). */
 YAS_API int yas_map_empty(yas_map *map, int *out_empty);
 /* MapStruct::Fuse(GpuMat depth, SE3d Tcm): VoxelMap.h:61 / VoxelMap.cu:825-884.
- * depth: float metres, `on_device` = 1 for a device pointer, 0 for host. */
+ * depth: float metres, `on_device` = 1 for a device pointer, 0 for host.  With a
+ * host depth the call returns once the map is fused; with a device pointer the
+ * fusion is enqueued on the map's stream. */
 YAS_API int yas_map_fuse_depth(yas_map *map, const float *depth, int width, int height,
                                int pitch_bytes, int on_device, const yas_pose *Tcm);
 /* MapStruct::CheckNumVisibleBlocks(cols, rows, Tcm): VoxelMap.h:59 / VoxelMap.cu:788-823. */

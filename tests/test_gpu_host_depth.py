@@ -1,10 +1,12 @@
-"""Fuse and Defuse of a host depth: rows that do not adjoin."""
+"""Fuse and Defuse of a host depth: rows that do not adjoin, and what has been done
+when the call returns."""
 from __future__ import annotations
 
 import ctypes as C
 
 import numpy as np
 import pytest
+import torch
 
 from yetanotherslam_gb300 import _lib as L
 from yetanotherslam_gb300 import rgbdfusion as rf
@@ -40,3 +42,17 @@ def test_padded_rows_fuse_as_adjoining_ones(cuda, w, h, pad):
         L.call(name, two.handle, room[at:].ctypes.data, w, h, 4 * (w + pad), 0, C.byref(T))
         for a, b in zip(_blocks(one), _blocks(two)):
             assert np.array_equal(a, b)
+
+
+def test_a_host_depth_is_fused_when_the_call_returns(cuda):
+    """The map's stream has nothing left to do: a program that reads the map on
+    another stream, or looks for an error, need not wait first."""
+    stream = torch.cuda.Stream()
+    w, h = 1280, 720
+    z = np.random.default_rng(3).uniform(0.8, 2.5, (h, w)).astype(np.float32)
+    m = _map((0.9 * w, 0.9 * w, (w - 1) / 2, (h - 1) / 2), stream.cuda_stream)
+    for _ in range(3):
+        m.Fuse(z, np.eye(4))
+        assert stream.query()
+        m.Defuse(z, np.eye(4))
+        assert stream.query()

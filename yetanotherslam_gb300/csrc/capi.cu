@@ -149,17 +149,6 @@ using namespace yas;
 // Per-map staging for host depth in yas_map_fuse_depth.
 struct MapExtra {
     Staging depth;
-    cudaEvent_t copied = nullptr;  // the caller's depth has been read
-    ~MapExtra() {
-        if (copied) cudaEventDestroy(copied);
-    }
-    int take(const float *src, size_t bytes, cudaStream_t s) {
-        YAS_TRY(depth.ensure(bytes));
-        if (!copied) YAS_TRY_CUDA(cudaEventCreateWithFlags(&copied, cudaEventDisableTiming));
-        YAS_TRY(copy_in(depth.ptr, src, bytes, s));
-        YAS_TRY_CUDA(cudaEventRecord(copied, s));
-        return YAS_OK;
-    }
 };
 static std::mutex g_extra_mutex;
 #include <unordered_map>
@@ -311,9 +300,11 @@ YAS_API int yas_map_fuse_depth(yas_map *m, const float *depth, int width, int he
         return YAS_ERR_BAD_ARG;
     if (m->hibernated) return YAS_ERR_STATE;
     const float *d = depth;
-    MapExtra *ex = on_device ? nullptr : map_extra(m);
-    if (ex) {
-        YAS_TRY(ex->take(depth, image_bytes((size_t)width * 4, (size_t)pitch_bytes, height), m->stream));
+    if (!on_device) {
+        MapExtra *ex = map_extra(m);
+        const size_t bytes = image_bytes((size_t)width * 4, (size_t)pitch_bytes, height);
+        YAS_TRY(ex->depth.ensure(bytes));
+        YAS_TRY(copy_in(ex->depth.ptr, depth, bytes, m->stream));
         d = (const float *)ex->depth.ptr;
     }
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, width, height);
@@ -324,8 +315,8 @@ YAS_API int yas_map_fuse_depth(yas_map *m, const float *depth, int width, int he
     launch_visible(v, cam, m->pose_dev, nullptr, m->stream, true);
     launch_integrate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, nullptr, m->stream, 0, true);
     YAS_TRY_CUDA(cudaGetLastError());
-    // the caller may write its depth again; the staging is reused in stream order
-    if (ex) YAS_TRY_CUDA(cudaEventSynchronize(ex->copied));
+    // a host depth: the caller may write it again, and the map is finished
+    if (!on_device) YAS_TRY_CUDA(cudaStreamSynchronize(m->stream));
     return YAS_OK;
 }
 
@@ -903,9 +894,11 @@ YAS_API int yas_map_defuse_depth(yas_map *m, const float *depth, int width, int 
         return YAS_ERR_BAD_ARG;
     if (m->hibernated) return YAS_ERR_STATE;
     const float *d = depth;
-    MapExtra *ex = on_device ? nullptr : map_extra(m);
-    if (ex) {
-        YAS_TRY(ex->take(depth, image_bytes((size_t)width * 4, (size_t)pitch_bytes, height), m->stream));
+    if (!on_device) {
+        MapExtra *ex = map_extra(m);
+        const size_t bytes = image_bytes((size_t)width * 4, (size_t)pitch_bytes, height);
+        YAS_TRY(ex->depth.ensure(bytes));
+        YAS_TRY(copy_in(ex->depth.ptr, depth, bytes, m->stream));
         d = (const float *)ex->depth.ptr;
     }
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, width, height);
@@ -914,7 +907,7 @@ YAS_API int yas_map_defuse_depth(yas_map *m, const float *depth, int width, int 
     launch_visible(v, cam, m->pose_dev, nullptr, m->stream, true);
     launch_deintegrate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, m->stream, true);
     YAS_TRY_CUDA(cudaGetLastError());
-    if (ex) YAS_TRY_CUDA(cudaEventSynchronize(ex->copied));
+    if (!on_device) YAS_TRY_CUDA(cudaStreamSynchronize(m->stream));
     return YAS_OK;
 }
 
