@@ -56,3 +56,16 @@ def test_a_host_depth_is_fused_when_the_call_returns(cuda):
         assert stream.query()
         m.Defuse(z, np.eye(4))
         assert stream.query()
+
+
+def test_a_call_that_fails_after_its_read_was_enqueued_waits_for_it(cuda):
+    """More rows than a launch's grid takes: the host refuses the allocation pass
+    when the depth's read is already under way."""
+    stream = torch.cuda.Stream()
+    w, h = 64, 8 * 65535 + 8
+    z = np.full((h, w), np.float32(0.5))
+    m = _map((0.9 * w, 0.9 * w, (w - 1) / 2, (h - 1) / 2), stream.cuda_stream)
+    m.Fuse(z[:8], np.eye(4))
+    with pytest.raises(L.YasError):
+        m.Fuse(z, np.eye(4))
+    assert stream.query()

@@ -763,7 +763,11 @@ YAS_API int yas_session_wait(yas_session *s, yas_pose *out_Tcm, int *out_status)
 
 YAS_API int yas_session_process_frame(yas_session *s, const uint8_t *rgb, const uint16_t *depth, int on_device,
                                       yas_pose *out_Tcm, int *out_status) {
-    YAS_TRY(yas_session_submit(s, rgb, depth, on_device));
+    const int st = yas_session_submit(s, rgb, depth, on_device);
+    if (st != YAS_OK) {
+        if (s) cudaStreamSynchronize(s->stream);  // nothing reads the caller's frame after the call
+        return st;
+    }
     return yas_session_wait(s, out_Tcm, out_status);
 }
 
