@@ -286,7 +286,10 @@ __device__ __forceinline__ float2 mix2(float2 a, float2 b, float t) {
     return cfma2(pair(1.0f - t), a, cmul2(pair(t), b));
 }
 
-// Reads of one ray.
+// Reads of one ray.  What the kernels of the same raycast write (grid, z-range
+// tiles) is read by plain loads: a march that starts beside the last of them
+// (dependent_wait) may not read it through the read-only path, which is for memory
+// that nothing writes while the kernel lasts.  Voxels and the table are older.
 template <int FMT>
 struct RayReader {
     typedef VoxelIO<FMT> IO;
@@ -298,14 +301,14 @@ struct RayReader {
     unsigned epoch;  // and its epoch << 24
 
     __device__ __forceinline__ RayReader(const MapDev &mm, const BlockGrid &gg)
-        : m(mm), g(gg), vox(static_cast<const V *>(mm.voxels)), ox(__ldg(gg.info)), oy(__ldg(gg.info + 1)),
-          oz(__ldg(gg.info + 2)), epoch((unsigned)__ldg(gg.info + 3) << 24) {}
+        : m(mm), g(gg), vox(static_cast<const V *>(mm.voxels)), ox(gg.info[0]), oy(gg.info[1]),
+          oz(gg.info[2]), epoch((unsigned)gg.info[3] << 24) {}
 
     // Pool index of block (x, y, z), or -1.
     __device__ __forceinline__ int lookup(int x, int y, int z) const {
         const int gx = x - ox, gy = y - oy, gz = z - oz;
         if (grid_holds(gx, gy, gz)) {
-            const unsigned w = __ldg(g.cells + grid_cell(gx, gy, gz)) - epoch;  // below 2^24 in this epoch only
+            const unsigned w = g.cells[grid_cell(gx, gy, gz)] - epoch;  // below 2^24 in this epoch only
             if (w != kGridAsk) return w < kGridAsk ? (int)w : -1;
         }
         return find_block_xyz(m, x, y, z);
@@ -344,7 +347,7 @@ struct RayReader {
             const int sx = across & 1u, sy = across & 2u ? kGridSide : 0, sz = across & 4u ? kGridSide * kGridSide : 0;
             lim = corner_blocks(
                 across, b, inner,
-                [&](unsigned c) { return __ldg(cell + ((c & 1 ? sx : 0) + (c & 2 ? sy : 0) + (c & 4 ? sz : 0))) - epoch; },
+                [&](unsigned c) { return cell[(c & 1 ? sx : 0) + (c & 2 ? sy : 0) + (c & 4 ? sz : 0)] - epoch; },
                 [&](unsigned d) { return lookup(bx + (int)(d & 1u), by + (int)((d >> 1) & 1u), bz + (int)(d >> 2)); }, q);
         }
         const int xo[2] = {x0 & 7, (x0 + 1) & 7}, yo[2] = {(y0 & 7) << 3, ((y0 + 1) & 7) << 3};
@@ -531,8 +534,8 @@ __device__ __forceinline__ float4 ray_finish(const RayReader<FMT> &rd, float rst
 constexpr float kLongBlocks = 16.0f;
 template <int FMT>
 __device__ __forceinline__ void march_pixel(const MapDev &m, const Cam &cam, const PosePair *P,
-                                            const float *__restrict__ znear, const float *__restrict__ zfar, int zw,
-                                            float4 *vmap, int vpitch, bool skipped, const float *__restrict__ fnear,
+                                            const float *znear, const float *zfar, int zw,
+                                            float4 *vmap, int vpitch, bool skipped, const float *fnear,
                                             int fw, const BlockGrid &g, int x, int y, int turn) {
     const float vsinv = 1.0f / m.voxel_size;
     const float rstep = m.trunc / m.voxel_size;
@@ -541,9 +544,9 @@ __device__ __forceinline__ void march_pixel(const MapDev &m, const Cam &cam, con
     R.sdf = 1.0f;
     float zn = 0.0f, zf = 0.0f, zfine = 0.0f;
     if (inside && !skipped) {
-        zn = __ldg(znear + (y >> 3) * zw + (x >> 3));
-        zf = __ldg(zfar + (y >> 3) * zw + (x >> 3));
-        zfine = __ldg(fnear + (y >> kFineShift) * fw + (x >> kFineShift));
+        zn = znear[(y >> 3) * zw + (x >> 3)];
+        zf = zfar[(y >> 3) * zw + (x >> 3)];
+        zfine = fnear[(y >> kFineShift) * fw + (x >> kFineShift)];
     }
     if (turn >= 0) {
         const bool far = zf - fmaxf(zn, zfine) > kLongBlocks * (float)kBlockSide * m.voxel_size;
@@ -565,10 +568,10 @@ __device__ __forceinline__ void march_pixel(const MapDev &m, const Cam &cam, con
 // lanes of a warp that jump, look up and sample take turns.
 template <int FMT, int WX, int WY, int RAYS>
 __global__ void __launch_bounds__(32 * WX * WY) march_kernel(MapDev m, Cam cam, const PosePair *P,
-                                                             const float *__restrict__ znear,
-                                                             const float *__restrict__ zfar, int zw, float4 *vmap,
+                                                             const float *znear,
+                                                             const float *zfar, int zw, float4 *vmap,
                                                              int vpitch, const int *skip,
-                                                             const float *__restrict__ fnear, int fw, BlockGrid g) {
+                                                             const float *fnear, int fw, BlockGrid g) {
     constexpr int TX = RAYS == 32 ? 8 : 4, TY = RAYS / TX;
     dependent_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -584,10 +587,10 @@ __global__ void __launch_bounds__(32 * WX * WY) march_kernel(MapDev m, Cam cam, 
 // same bit for bit.
 template <int FMT>
 __global__ void __launch_bounds__(128) march_persistent_kernel(MapDev m, Cam cam, const PosePair *P,
-                                                               const float *__restrict__ znear,
-                                                               const float *__restrict__ zfar, int zw, float4 *vmap,
+                                                               const float *znear,
+                                                               const float *zfar, int zw, float4 *vmap,
                                                                int vpitch, const int *skip,
-                                                               const float *__restrict__ fnear, int fw,
+                                                               const float *fnear, int fw,
                                                                BlockGrid g, unsigned *queue,
                                                                unsigned tiles) {
     const int lane = (int)lane_id(), tiles_x = (cam.w + 7) >> 3;
