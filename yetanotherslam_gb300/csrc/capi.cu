@@ -294,7 +294,6 @@ YAS_API int yas_map_destroy(yas_map *m) {
 YAS_API int yas_map_reset(yas_map *m) {
     if (!m) return YAS_ERR_BAD_ARG;
     if (m->hibernated) return YAS_ERR_STATE;
-    m->edits++;
     launch_map_reset(map_view(m), m->stream);
     YAS_TRY_CUDA(cudaGetLastError());
     return YAS_OK;
@@ -333,7 +332,7 @@ YAS_API int yas_map_fuse_depth(yas_map *m, const float *depth, int width, int he
     }
     Cam cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, width, height);
     MapDev v = map_view(m);
-    m->edits++;
+    m->additions++;
     launch_pose_begin(v, make_pair(Tcm), m->pose_dev, m->stream);
     launch_allocate(v, m->cfg.voxel_format, d, pitch_bytes / 4, cam, m->pose_dev, nullptr, m->stream, true);
     launch_visible(v, cam, m->pose_dev, nullptr, m->stream, true);
@@ -451,7 +450,7 @@ YAS_API int yas_map_import(yas_map *m, const int *coords, const float *sdf, cons
         cudaFree(dw);
         return YAS_ERR_OOM;
     }
-    m->edits++;
+    m->additions++;
     int st = YAS_OK;
     if (cudaMemcpyAsync(dc, coords, (size_t)count * 12, cudaMemcpyHostToDevice, m->stream) != cudaSuccess ||
         cudaMemcpyAsync(ds, sdf, (size_t)count * 2048, cudaMemcpyHostToDevice, m->stream) != cudaSuccess ||
@@ -698,7 +697,6 @@ YAS_API int yas_map_load(yas_map *m, const char *path) {
         YAS_TRY_CUDA(cudaMemcpyAsync(m->voxels, vox.data(), vox.size(), cudaMemcpyHostToDevice, m->stream));
         YAS_TRY_CUDA(cudaMemcpyAsync(&m->hdr->n_alloc, &n, sizeof(unsigned), cudaMemcpyHostToDevice, m->stream));
         launch_rehash(map_view(m), n, m->stream);
-        m->edits++;
         YAS_TRY_CUDA(cudaGetLastError());
     }
     YAS_TRY(read_header(m));
@@ -773,8 +771,6 @@ static void swap_storage(yas_map *a, yas_map *b) {
     std::swap(a->hib_voxels, b->hib_voxels);
     std::swap(a->hib_visible, b->hib_visible);
     std::swap(a->hib_hdr, b->hib_hdr);
-    a->edits++;
-    b->edits++;
 }
 
 static int map_grow(yas_map *m, long long want_slots, long long want_blocks) {
@@ -882,7 +878,6 @@ YAS_API int yas_map_fuse_map(yas_map *dst, yas_map *src) {
     YAS_TRY(map_grow(dst, 2 * want_blocks, want_blocks));
     YAS_TRY_CUDA(cudaMemsetAsync(&dst->hdr->err_bits, 0, sizeof(unsigned), dst->stream));
     YAS_TRY_CUDA(cudaStreamSynchronize(src->stream));
-    dst->edits++;
     for (int attempt = 0;; ++attempt) {
         launch_fuse_alloc(map_view(dst), map_view(src), dst->cfg.voxel_format, T_src_dst, nsrc, dst->stream);
         YAS_TRY_CUDA(cudaGetLastError());

@@ -11,6 +11,8 @@
 // voxel pool is bump-allocated so pool index i <-> block_keys[i] is itself
 // the allocated-block list (no full-table scans); new blocks are zeroed by the
 // warp that allocated them.
+#include <atomic>
+
 #include "yas_internal.h"
 
 namespace yas {
@@ -429,7 +431,7 @@ void launch_deintegrate(const MapDev &m, int fmt, const float *depth, int pitch_
 }
 
 // ---------------------------------------------------------------- reset
-__global__ void reset_slots_kernel(MapDev m) {
+__global__ void reset_slots_kernel(MapDev m, unsigned block_set) {
     const unsigned n = m.slot_mask + 1;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         HashSlot s;
@@ -440,12 +442,16 @@ __global__ void reset_slots_kernel(MapDev m) {
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         MapHeader h = {};
+        h.block_set = block_set;
         *m.hdr = h;
     }
 }
 
 void launch_map_reset(const MapDev &m, cudaStream_t s) {
-    reset_slots_kernel<<<kSMs * 4, 256, 0, s>>>(m);
+    static std::atomic<unsigned> drawn{0};
+    unsigned block_set = ++drawn;
+    if (block_set == 0u) block_set = ++drawn;
+    reset_slots_kernel<<<kSMs * 4, 256, 0, s>>>(m, block_set);
 }
 
 // ---------------------------------------------------------------- export/import

@@ -150,7 +150,10 @@ struct __align__(16) MapHeader {
     unsigned n_visible;     // length of the visible list
     unsigned err_bits;      // sticky yas_status bits
     unsigned n_alloc_prev;  // n_alloc before the latest allocation pass
-    unsigned pad[4];
+    // Drawn anew at every reset, never 0.  Between resets the pool only grows and a
+    // block keeps its index, so (block_set, n_alloc) names the set of blocks.
+    unsigned block_set;
+    unsigned pad[3];
 };
 
 // ------------------------------------------------------------------ formats

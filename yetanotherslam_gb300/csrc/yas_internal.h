@@ -116,7 +116,7 @@ void launch_visible_coords(const MapDev &m, int *coords, unsigned count, cudaStr
 // The blocks around a raycast's view (raycast.cu).
 struct BlockGrid {
     unsigned *cells;  // pool index of each block, tagged with the epoch
-    int *info;        // first block and epochs
+    int *info;        // first block, epochs, the block set it shows
 };
 struct RaycastBuffers {
     int w, h;          // image size
@@ -131,18 +131,18 @@ struct RaycastBuffers {
 int raycast_buffers_alloc(RaycastBuffers &rb, int width, int height);
 void raycast_buffers_free(RaycastBuffers &rb);
 // Z-range tiles of the visible list and the block grid of the allocated blocks,
-// for a march at the same pose.
+// for a march at the same pose; blocks that the map gains or loses before it are
+// seen (the march then leaves the grid aside).
 void launch_zrange(const MapDev &m, const Cam &cam, const PosePair *P, RaycastBuffers &rb,
                    const int *skip, cudaStream_t s);
+// The block grid alone, after blocks were added between launch_zrange and the march.
+void launch_block_grid(const MapDev &m, const PosePair *P, const RaycastBuffers &rb, cudaStream_t s);
 // A raycast at a pose given by the host: the pose into *P, visibility (vis_cam),
 // z-range tiles, block grid and march, each a programmatic dependent of the one
 // before.  The length of the visible list also goes to *host_visible (mapped
 // host memory).
 void launch_raycast(const MapDev &m, int fmt, const Cam &vis_cam, const Cam &cam, const PosePair &pose, PosePair *P,
                     RaycastBuffers &rb, float4 *vmap, int vmap_pitch_elems, unsigned *host_visible, cudaStream_t s);
-// The block grid alone, for a map whose blocks changed between launch_zrange
-// and the march.
-void launch_block_grid(const MapDev &m, const PosePair *P, const RaycastBuffers &rb, cudaStream_t s);
 // `warps_x` 1, 2 (the default), 4: one thread per pixel, a 128-thread CTA's
 // four 8x4-pixel warp tiles side by side in x (8x16, 16x8, 32x4 pixels);
 // 0: persistent warps taking 8x4-pixel tiles from a queue.  The output is
@@ -191,9 +191,9 @@ struct yas_map {
     std::mutex pose_mutex;
     bool active = true;
     std::mutex active_mutex;
-    // counts the calls that may have changed the block set outside a session's
-    // frames: a session's next raycast looks blocks up in a grid made before
-    std::atomic<unsigned long long> edits{0};
+    // counts the calls that may have added a few blocks (Fuse, import): a hint to a
+    // session that its next raycast is faster with a new block grid
+    std::atomic<unsigned long long> additions{0};
     bool hibernated = false;
     std::vector<unsigned char> hib_slots, hib_keys, hib_voxels, hib_visible;
     yas::MapHeader hib_hdr;
