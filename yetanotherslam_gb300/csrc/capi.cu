@@ -979,6 +979,7 @@ YAS_API int yas_raycaster_raycast(yas_raycaster *rc, yas_map *m, const yas_pose 
     // The map's stream may differ: order the map's pending work first.
     if (m->stream != s) YAS_TRY_CUDA(cudaStreamSynchronize(m->stream));
     Cam vis_cam = make_cam(m->cam_K.fx, m->cam_K.fy, m->cam_K.cx, m->cam_K.cy, rc->w, rc->h);
+    block_grid_alloc(rc->rb.grid);  // the first raycast's: a raycaster that makes none (a session's own) does without
     launch_raycast(map_view(m), m->cfg.voxel_format, vis_cam, rc->cam, make_pair(Tcm), rc->pose_dev, rc->rb, rc->vmap,
                    rc->w, rc->visible_dev, s);
     YAS_TRY_CUDA(cudaGetLastError());

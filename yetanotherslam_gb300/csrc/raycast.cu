@@ -56,15 +56,14 @@ namespace yas {
 // front of the cells, kept by the ray per 4x4x4 blocks, saved reads but cost
 // more in instructions: 174 against 161 us at 1280x720, 4 mm.)  Blocks outside
 // the grid, and those whose index does not fit 24 bits (kGridAsk), are looked
-// up in the table.
+// up in the table; all of them where there is no grid (no memory for one).
 // info: first block x, y, z; epoch; epoch of the next raycast; the map's block_set
-// and block count when it was filled.  A march that finds another set in the map,
+// and n_alloc when it was filled.  A march that finds another set in the map,
 // as after an import, a Fuse or a reset between a session's frames, looks all its
 // blocks up in the table: the comparison is made on the GPU, in the stream's order,
 // whoever changed the map (640x480, 5 mm, a frame after a block was imported: 456 us
 // by the table, 425 by a new grid).
-
-constexpr int kGridInfo = 7;
+constexpr int kGridInfo = 8;
 
 __device__ __forceinline__ int grid_cell(int x, int y, int z) { return (z * kGridSide + y) * kGridSide + x; }
 __device__ __forceinline__ bool grid_holds(int x, int y, int z) {
@@ -74,6 +73,7 @@ __device__ __forceinline__ bool grid_holds(int x, int y, int z) {
 // Opens an epoch: the grid is centred half way along the depth range, at most
 // 64 blocks ahead of the camera.  (grid_fill, the next kernel, writes info[4].)
 __device__ __forceinline__ void grid_begin(const MapDev &m, const Rigid32 &T, const BlockGrid &g) {
+    if (!g.cells) return;
     const int next = g.info[4], epoch = next < 1 || next > 255 ? 1 : next;
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     if (epoch == 1)
@@ -92,6 +92,7 @@ __device__ __forceinline__ void grid_begin(const MapDev &m, const Rigid32 &T, co
 }
 
 __device__ __forceinline__ void grid_fill(const MapDev &m, const BlockGrid &g) {
+    if (!g.cells) return;
     const int ox = g.info[0], oy = g.info[1], oz = g.info[2];
     const unsigned epoch = (unsigned)g.info[3] << 24, n = num_blocks(m);
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -103,7 +104,7 @@ __device__ __forceinline__ void grid_fill(const MapDev &m, const BlockGrid &g) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         g.info[4] = g.info[3] + 1;
         g.info[5] = (int)m.hdr->block_set;
-        g.info[6] = (int)n;
+        g.info[6] = (int)m.hdr->n_alloc;
     }
 }
 
@@ -224,6 +225,13 @@ __global__ void __launch_bounds__(128) zrange_fill_kernel(MapDev m, Cam cam, con
     }
 }
 
+// No epoch and no block set: the next raycast clears the cells.  (The fill runs on
+// the legacy stream, which the raycaster's non-blocking stream does not wait for.)
+static bool grid_forget(const BlockGrid &g) {
+    return cudaMemset(g.info, 0, kGridInfo * sizeof(int)) == cudaSuccess &&
+           cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess;
+}
+
 int raycast_buffers_alloc(RaycastBuffers &rb, int width, int height) {
     rb.w = width;
     rb.h = height;
@@ -235,17 +243,27 @@ int raycast_buffers_alloc(RaycastBuffers &rb, int width, int height) {
     if (cudaMalloc(&rb.znear, nz * 4) != cudaSuccess || cudaMalloc(&rb.zfar, nz * 4) != cudaSuccess ||
         cudaMalloc(&rb.queue, sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc(&rb.fnear, (size_t)rb.fw * rb.fh * 4) != cudaSuccess ||
-        cudaMalloc(&rb.grid.cells, kGridCells * sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc(&rb.grid.info, kGridInfo * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         return YAS_ERR_OOM;
     }
-    // no epoch yet: the first raycast clears the cells.  The fill runs on the
-    // legacy stream, which the raycaster's non-blocking stream does not wait for
-    if (cudaMemset(rb.grid.info, 0, kGridInfo * sizeof(int)) != cudaSuccess ||
-        cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)
-        return YAS_ERR_CUDA;
-    return YAS_OK;
+    return grid_forget(rb.grid) ? YAS_OK : YAS_ERR_CUDA;
+}
+
+void block_grid_alloc(BlockGrid &g) {
+    if (g.cells) return;
+    unsigned *cells = nullptr;
+    if (cudaMalloc(&cells, kGridBytes) != cudaSuccess || !grid_forget(g)) {
+        cudaGetLastError();
+        cudaFree(cells);
+        return;
+    }
+    g.cells = cells;
+}
+
+void block_grid_free(BlockGrid &g) {
+    cudaFree(g.cells);
+    g.cells = nullptr;
 }
 
 void raycast_buffers_free(RaycastBuffers &rb) {
@@ -313,12 +331,15 @@ struct RayReader {
     unsigned epoch;  // and its epoch << 24
 
     __device__ __forceinline__ RayReader(const MapDev &mm, const BlockGrid &gg)
-        : m(mm), g(gg), vox(static_cast<const V *>(mm.voxels)),
-          ox(gg.info[5] == (int)mm.hdr->block_set && gg.info[6] == (int)min(mm.hdr->n_alloc, (unsigned)mm.max_blocks)
-                 ? gg.info[0]
-                 : INT_MIN / 2),
-          oy(gg.info[1]),
-          oz(gg.info[2]), epoch((unsigned)gg.info[3] << 24) {}
+        : m(mm), g(gg), vox(static_cast<const V *>(mm.voxels)) {
+        const int4 at = reinterpret_cast<const int4 *>(gg.info)[0], of = reinterpret_cast<const int4 *>(gg.info)[1];
+        const uint2 now = *reinterpret_cast<const uint2 *>(mm.hdr);  // n_alloc, block_set
+        const bool same = gg.cells && (unsigned)of.z == now.x && (unsigned)of.y == now.y;
+        ox = same ? at.x : INT_MIN / 2;
+        oy = at.y;
+        oz = at.z;
+        epoch = (unsigned)at.w << 24;
+    }
 
     // Pool index of block (x, y, z), or -1.
     __device__ __forceinline__ int lookup(int x, int y, int z) const {

@@ -91,8 +91,7 @@ size_t session_bytes_estimate(const yas_session_config &c) {
     const size_t P0 = (size_t)c.width * c.height;
     const size_t pyramids = 88 * P;                       // two frame sets + gradients
     const size_t frame = P0 * (16 + 4 + 16 + 4 + 3 + 2 + 4); // residuals, staging, vmap, depth, inputs
-    const size_t grids = 2 * (size_t)kGridCells * 4;      // block grids of the frames' raycast and the raycaster
-    return map + pyramids + frame + grids + (8u << 20);   // + tracker rows, graphs, small buffers
+    return map + pyramids + frame + (8u << 20);            // + tracker rows, graphs, small buffers
 }
 
 }  // namespace
@@ -388,6 +387,24 @@ YAS_API int yas_server_create(yas_server **out, const yas_server_config *cfg) {
     return YAS_OK;
 }
 
+// Free device memory, at least `need` of it if that is to be had: where it is short
+// the sessions' block grids go first, so that they make nobody wait or be refused.
+static int free_memory(yas_server *srv, size_t need, size_t *out) {
+    size_t total = 0;
+    YAS_TRY_CUDA(cudaMemGetInfo(out, &total));
+    if (*out >= need) return YAS_OK;
+    {
+        std::unique_lock<std::mutex> lk(srv->mu);
+        for (size_t i = 0; i < srv->sessions.size(); ++i) {
+            // (the worker starts a frame with the lock held)
+            srv->cv.wait(lk, [&] { return !srv->sessions[i] || !srv->sessions[i]->in_flight || srv->stop.load(); });
+            if (srv->sessions[i] && !srv->sessions[i]->in_flight) session_drop_grid(srv->sessions[i]->s);
+        }
+    }
+    YAS_TRY_CUDA(cudaMemGetInfo(out, &total));
+    return YAS_OK;
+}
+
 YAS_API int yas_server_open_session(yas_server *srv, const yas_session_config *cfg, int *out_id) {
     if (!srv || !cfg || !out_id || cfg->width <= 0 || cfg->height <= 0) return YAS_ERR_BAD_ARG;
     static std::mutex open_mu;  // admission decisions one at a time
@@ -399,11 +416,15 @@ YAS_API int yas_server_open_session(yas_server *srv, const yas_session_config *c
         if (live >= srv->cfg.max_sessions) return YAS_ERR_CAPACITY;
     }
     cudaSetDevice(srv->device);
-    size_t free_b = 0, total_b = 0;
-    YAS_TRY_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    if (free_b < session_bytes_estimate(*cfg) + srv->cfg.hbm_reserve_bytes) return YAS_ERR_OOM;  // not admitted
+    const size_t need = session_bytes_estimate(*cfg) + srv->cfg.hbm_reserve_bytes;
+    size_t free_b = 0;
+    YAS_TRY(free_memory(srv, need, &free_b));
+    if (free_b < need) return YAS_ERR_OOM;  // not admitted
     ServedSession *ss = new ServedSession();
-    int st = yas_session_create(&ss->s, cfg, nullptr);
+    // its raycasts are faster with a block grid, which is no reason to refuse it
+    const bool grid = free_b - need >= kGridBytes;
+    int st = session_create(&ss->s, cfg, nullptr, grid);
+    if (st == YAS_ERR_OOM && grid) st = session_create(&ss->s, cfg, nullptr, false);
     ss->w = cfg->width;
     ss->h = cfg->height;
     ss->ring = srv->cfg.ring_frames;
@@ -472,10 +493,10 @@ YAS_API int yas_server_resume_session(yas_server *srv, int id) {
     yas_map *m = nullptr;
     YAS_TRY(yas_session_map(ss->s, &m));
     // admission: the map's arrays must fit the free HBM minus the reserve
-    size_t free_b = 0, total_b = 0;
-    YAS_TRY_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t vb = m->cfg.voxel_format == YAS_VOXEL_F32 ? 8 : 4;
     const size_t need = (size_t)m->cfg.hash_slots * sizeof(HashSlot) + (size_t)m->cfg.max_blocks * (12 + kBlockVoxels * vb);
+    size_t free_b = 0;
+    YAS_TRY(free_memory(srv, need + srv->cfg.hbm_reserve_bytes, &free_b));
     if (free_b < need + srv->cfg.hbm_reserve_bytes) return YAS_ERR_OOM;
     YAS_TRY(yas_map_reactivate(m));
     {

@@ -620,8 +620,18 @@ YAS_API int yas_session_config_default(yas_session_config *cfg, int width, int h
 
 YAS_API int yas_session_destroy(yas_session *s);
 
-YAS_API int yas_session_create(yas_session **out, const yas_session_config *cfg, void *stream) {
-    if (!out || !cfg || cfg->width <= 0 || cfg->height <= 0) return YAS_ERR_BAD_ARG;
+}  // extern "C"
+
+namespace yas {
+
+void session_drop_grid(yas_session *s) {
+    if (!s->zt.grid.cells) return;
+    cudaStreamSynchronize(s->stream);
+    drop_graphs(s);  // they name the cells
+    block_grid_free(s->zt.grid);
+}
+
+int session_create(yas_session **out, const yas_session_config *cfg, void *stream, bool block_grid) {
     *out = nullptr;
     yas_session *s = new yas_session();
     s->cfg = *cfg;
@@ -648,6 +658,7 @@ YAS_API int yas_session_create(yas_session **out, const yas_session_config *cfg,
     int st = yas_map_create(&s->map, &cfg->map, &cfg->K, s->stream);
     if (st == YAS_OK) st = yas_raycaster_create(&s->rc, cfg->width, cfg->height, &cfg->K, s->stream);
     if (st == YAS_OK) st = raycast_buffers_alloc(s->zt, cfg->width, cfg->height);
+    if (st == YAS_OK && block_grid) block_grid_alloc(s->zt.grid);
     if (st == YAS_OK) {
         const double K[9] = {cfg->K.fx, 0, cfg->K.cx, 0, cfg->K.fy, cfg->K.cy, 0, 0, 1};
         st = yas_tracker_create(&s->tr, cfg->width, cfg->height, K, cfg->num_levels, cfg->iterations, cfg->mode,
@@ -684,6 +695,16 @@ YAS_API int yas_session_create(yas_session **out, const yas_session_config *cfg,
     }
     *out = s;
     return YAS_OK;
+}
+
+}  // namespace yas
+
+extern "C" {
+
+YAS_API int yas_session_create(yas_session **out, const yas_session_config *cfg, void *stream) {
+    if (!out || !cfg || cfg->width <= 0 || cfg->height <= 0) return YAS_ERR_BAD_ARG;
+    const int st = session_create(out, cfg, stream, true);
+    return st == YAS_ERR_OOM ? session_create(out, cfg, stream, false) : st;
 }
 
 YAS_API int yas_session_destroy(yas_session *s) {

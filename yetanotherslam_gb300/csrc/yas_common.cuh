@@ -30,9 +30,12 @@ constexpr int kSMs = 152;
 // Fine near-bound cells of the ray march: 2^kFineShift pixels square.
 constexpr int kFineShift = 2;
 // Block grid of a raycast: blocks per side, blocks.  160 blocks span the 3 m
-// view frustum in any orientation at 5 mm voxels and most of it at 4 mm.
+// view frustum in any orientation at 5 mm voxels and most of it at 4 mm; coarser
+// voxels would do with fewer, but a side that is not a constant costs the march 2
+// to 4% (640x480, 5 mm 90 / 93 us, 1280x720, 4 mm 201 / 209).
 constexpr int kGridSide = 160;
 constexpr int kGridCells = kGridSide * kGridSide * kGridSide;
+constexpr size_t kGridBytes = (size_t)kGridCells * sizeof(unsigned);  // 16.4 MB
 constexpr int kCoordBits = 21;
 constexpr int kCoordMax = (1 << (kCoordBits - 1)) - 1;   // 1048575
 constexpr int kCoordMin = -(1 << (kCoordBits - 1));      // -1048576
@@ -147,12 +150,12 @@ struct __align__(16) HashSlot {
 // Device-resident counters of one map.
 struct __align__(16) MapHeader {
     unsigned n_alloc;       // bump counter of the block pool (may pass max_blocks on overflow)
+    // Drawn anew at every reset, never 0.  Between resets the pool only grows and a
+    // block keeps its index, so (n_alloc, block_set) names the set of blocks.
+    unsigned block_set;
     unsigned n_visible;     // length of the visible list
     unsigned err_bits;      // sticky yas_status bits
     unsigned n_alloc_prev;  // n_alloc before the latest allocation pass
-    // Drawn anew at every reset, never 0.  Between resets the pool only grows and a
-    // block keeps its index, so (block_set, n_alloc) names the set of blocks.
-    unsigned block_set;
     unsigned pad[3];
 };
 

@@ -113,7 +113,8 @@ void launch_map_import(const MapDev &m, int fmt, const int *coords, const float 
 void launch_visible_coords(const MapDev &m, int *coords, unsigned count, cudaStream_t s);
 
 // ------------------------------------------------------------------ raycast.cu
-// The blocks around a raycast's view (raycast.cu).
+// The blocks around a raycast's view (raycast.cu); without cells where there was no
+// memory for them.
 struct BlockGrid {
     unsigned *cells;  // pool index of each block, tagged with the epoch
     int *info;        // first block, epochs, the block set it shows
@@ -128,7 +129,11 @@ struct RaycastBuffers {
     float *fnear;      // fw*fh: nearest visible block whose projected box covers the 4x4 pixels
     BlockGrid grid;
 };
-int raycast_buffers_alloc(RaycastBuffers &rb, int width, int height);
+int raycast_buffers_alloc(RaycastBuffers &rb, int width, int height);  // without a block grid
+// Cells for the grid, if it has none and there is memory; and gives them back (no
+// kernel that uses them may be in flight).
+void block_grid_alloc(BlockGrid &g);
+void block_grid_free(BlockGrid &g);
 void raycast_buffers_free(RaycastBuffers &rb);
 // Z-range tiles of the visible list and the block grid of the allocated blocks,
 // for a march at the same pose; blocks that the map gains or loses before it are

@@ -20,6 +20,11 @@ struct LaunchShape {
     int gn_pixels_per_cta = 32768;  // batched GN: one CTA per this many level-0 pixels
 };
 
+// yas_session_create for arguments that were looked at; without its block grid, the
+// session's raycasts look blocks up in the hash table (the same results, slower).
+int session_create(yas_session **out, const yas_session_config *cfg, void *stream, bool block_grid);
+// Gives the block grid's memory back (no frame of the session may be in flight).
+void session_drop_grid(yas_session *s);
 // Copies one frame (RGB u8 interleaved, depth u16) into the session's device
 // buffers on its stream.
 int session_copy_input(yas_session *s, const uint8_t *rgb, const uint16_t *depth, int on_device);
