@@ -47,12 +47,14 @@ namespace yas {
 
 // Block grid of a raycast: a cell for each of the kGridSide^3 blocks around the
 // middle of the view, which rays look their blocks up in instead of the hash
-// table.  A cell holds epoch << 24 | pool index; one of an earlier epoch is an
-// unallocated block, so cells are cleared only when the epoch wraps (every
-// 255th raycast).  Most lookups of a long ray are of unallocated blocks (59 of
-// 74 samples of the longest 2000 rays at 640x480, 5 mm): in the table each a
-// 64-bit hash and a read of a random line of 16-32 MB, here a few index
-// instructions and a line that neighbouring rays share.  (A bit per block in
+// table.  A cell holds epoch << 24 | pool index; one of another epoch is an
+// unallocated block.  Raycast e of the 255 epochs clears slice e of the cells before
+// it fills its own, so that none keeps an epoch until that comes again (all of them
+// at once, every 255th raycast of 160x120 took 107 us instead of 57).
+// Most lookups of a long ray are of unallocated blocks (59 of 74 samples of the
+// longest 2000 rays at 640x480, 5 mm): in the table each a 64-bit hash and a read
+// of a random line of 16-32 MB, here a few index instructions and a line that
+// neighbouring rays share.  (A bit per block in
 // front of the cells, kept by the ray per 4x4x4 blocks, saved reads but cost
 // more in instructions: 174 against 161 us at 1280x720, 4 mm.)  Blocks outside
 // the grid, and those whose index does not fit 24 bits (kGridAsk), are looked
@@ -64,6 +66,8 @@ namespace yas {
 // whoever changed the map (640x480, 5 mm, a frame after a block was imported: 456 us
 // by the table, 425 by a new grid).
 constexpr int kGridInfo = 8;
+constexpr int kGridEpochs = 255;
+constexpr int kGridSlice = (kGridCells / 4 + kGridEpochs - 1) / kGridEpochs;  // 16-byte words
 
 __device__ __forceinline__ int grid_cell(int x, int y, int z) { return (z * kGridSide + y) * kGridSide + x; }
 __device__ __forceinline__ bool grid_holds(int x, int y, int z) {
@@ -74,11 +78,11 @@ __device__ __forceinline__ bool grid_holds(int x, int y, int z) {
 // 64 blocks ahead of the camera.  (grid_fill, the next kernel, writes info[4].)
 __device__ __forceinline__ void grid_begin(const MapDev &m, const Rigid32 &T, const BlockGrid &g) {
     if (!g.cells) return;
-    const int next = g.info[4], epoch = next < 1 || next > 255 ? 1 : next;
+    const int next = g.info[4], epoch = next < 1 || next > kGridEpochs ? 1 : next;
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-    if (epoch == 1)
-        for (int i = i0; i < kGridCells / 4; i += stride)
-            reinterpret_cast<uint4 *>(g.cells)[i] = make_uint4(0u, 0u, 0u, 0u);
+    const int end = min(epoch * kGridSlice, kGridCells / 4);
+    for (int i = (epoch - 1) * kGridSlice + i0; i < end; i += stride)
+        reinterpret_cast<uint4 *>(g.cells)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (i0 == 0) {
         const float side = m.voxel_size * (float)kBlockSide;
         const float3 c = rigid_fast(T, 0.0f, 0.0f, fminf(0.5f * m.depth_max, 64.0f * side));
@@ -225,7 +229,7 @@ __global__ void __launch_bounds__(128) zrange_fill_kernel(MapDev m, Cam cam, con
     }
 }
 
-// No epoch and no block set: the next raycast clears the cells.  (The fill runs on
+// No epoch and no block set: the next raycast begins with epoch 1.  (The fill runs on
 // the legacy stream, which the raycaster's non-blocking stream does not wait for.)
 static bool grid_forget(const BlockGrid &g) {
     return cudaMemset(g.info, 0, kGridInfo * sizeof(int)) == cudaSuccess &&
@@ -253,7 +257,8 @@ int raycast_buffers_alloc(RaycastBuffers &rb, int width, int height) {
 void block_grid_alloc(BlockGrid &g) {
     if (g.cells) return;
     unsigned *cells = nullptr;
-    if (cudaMalloc(&cells, kGridBytes) != cudaSuccess || !grid_forget(g)) {
+    if (cudaMalloc(&cells, kGridBytes) != cudaSuccess || cudaMemset(cells, 0, kGridBytes) != cudaSuccess ||
+        !grid_forget(g)) {
         cudaGetLastError();
         cudaFree(cells);
         return;
@@ -279,7 +284,7 @@ void raycast_buffers_free(RaycastBuffers &rb) {
 void launch_zrange(const MapDev &m, const Cam &cam, const PosePair *P, RaycastBuffers &rb,
                    const int *skip, cudaStream_t s) {
     const int n = rb.zw * rb.zh, nf = rb.fw * rb.fh;
-    zrange_reset_kernel<<<(std::max(n, nf) + 255) / 256, 256, 0, s>>>(m, P, rb.znear, rb.zfar, n, rb.queue, rb.fnear,
+    zrange_reset_kernel<<<(std::max({n, nf, kGridSlice}) + 255) / 256, 256, 0, s>>>(m, P, rb.znear, rb.zfar, n, rb.queue, rb.fnear,
                                                                       nf, rb.grid);
     zrange_fill_kernel<<<kSMs * 8, 128, 0, s>>>(m, cam, P, rb.znear, rb.zfar, rb.zw, rb.zh, skip, rb.fnear, rb.fw,
                                                rb.fh, rb.grid, nullptr);
@@ -743,7 +748,7 @@ void launch_march(const MapDev &m, int fmt, const Cam &cam, const PosePair *P, c
 void launch_raycast(const MapDev &m, int fmt, const Cam &vis_cam, const Cam &cam, const PosePair &pose, PosePair *P,
                     RaycastBuffers &rb, float4 *vmap, int vmap_pitch_elems, unsigned *host_visible, cudaStream_t s) {
     const int n = rb.zw * rb.zh, nf = rb.fw * rb.fh;
-    raycast_begin_kernel<<<(std::max(n, nf) + 255) / 256, 256, 0, s>>>(m, pose, P, rb.znear, rb.zfar, n, rb.queue,
+    raycast_begin_kernel<<<(std::max({n, nf, kGridSlice}) + 255) / 256, 256, 0, s>>>(m, pose, P, rb.znear, rb.zfar, n, rb.queue,
                                                                        rb.fnear, nf, rb.grid);
     launch_visible(m, vis_cam, P, nullptr, s, true);
     launch_kernel(zrange_fill_kernel, dim3(kSMs * 8), dim3(128), s, true, m, cam, (const PosePair *)P, rb.znear, rb.zfar,
