@@ -17,6 +17,8 @@
 // Triangles with a vertex nearer than 5 cm are not drawn (no clipping).
 // All arithmetic is one rounding per operation in a fixed order, so the image
 // is reproducible bit for bit by a CPU restatement.
+#include <mutex>
+
 #include "yas_internal.h"
 
 struct yas_canvas {
@@ -28,6 +30,7 @@ struct yas_canvas {
     // allocated for one read goes back to the system at its synchronisation, and
     // a 640x480 read took 213 us for the 45 that its copies take.
     uchar4 *image = nullptr;
+    std::mutex image_mutex;  // one host read at a time: its colours and depths are of one moment
 };
 
 namespace yas {
@@ -333,6 +336,8 @@ YAS_API int yas_canvas_read(yas_canvas *c, uint8_t *rgba, int rgba_pitch, float 
         drgba = rgba ? c->image : nullptr;
         ddepth = depth ? reinterpret_cast<float *>(c->image + (size_t)c->w * c->h) : nullptr;
     }
+    std::unique_lock<std::mutex> lk(c->image_mutex, std::defer_lock);
+    if (!on_device) lk.lock();
     const int rp = on_device ? rgba_pitch / 4 : c->w, dp = on_device ? depth_pitch / 4 : c->w;
     dim3 grid((c->w + 31) / 32, (c->h + 7) / 8);
     canvas_resolve_kernel<<<grid, dim3(32, 8), 0, c->stream>>>(c->keys, c->w, c->h, drgba, rp, ddepth, dp);
