@@ -216,9 +216,10 @@ static int plan_gn(yas_batch *b, const std::vector<uint8_t> &key, std::vector<GN
 }
 
 // Sessions from which on a step's raycasts fill the GPU beside one another
-// (steps of mixed sessions with the march's warps as for a shared GPU and as
-// for a lone one: one session 286 and 282 us, three 548 and 546, four 628 and
-// 638, eight 1251 and 1272).
+// (steps of mixed sessions with the march's warps as for a lone GPU and as for a
+// shared one, medians of three runs, each within 1 %: one session 295 / 301 us, two
+// 486 / 488, three 575 / 572, four 655 / 645, five 832 / 819, six 978 / 962, eight
+// 1277 / 1243; at three the two are not told apart).
 constexpr size_t kSharedSessions = 4;
 
 static int capture_step(yas_batch *b, const std::vector<uint8_t> &key, CachedStep &out) {

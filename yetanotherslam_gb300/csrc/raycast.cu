@@ -718,12 +718,22 @@ static void launch_march_tile(const MapDev &m, int fmt, const Cam &cam, const Po
                               bool dependent = false, bool shared = false) {
     // Rays per warp.  A small image does not fill the GPU with warps of 32 rays,
     // so a march lasts as long as its slowest warp, and that one ends sooner
-    // with fewer rays: 320x240, 8 mm: 56 us at 32 rays, 50 at 16 and 49 at 8;
-    // 160x120, 1 cm: 51 at 32 and 38 at 8.  In larger images instruction issue
-    // counts, and full warps take the fewest: 640x480, 5 mm: 79 us at 32, 96 at
-    // 16, 149 at 8.  So they do where the marches of several sessions fill the GPU.
-    const int px = cam.w * cam.h;
-    if (px <= 40000 && !shared)
+    // with fewer rays; in larger images instruction issue counts, and full warps
+    // take the fewest.  Whole raycasts with 8 / 16 / 32 rays a warp (us, means of
+    // three scenes of four frames, the smaller of two runs each):
+    //               8 mm F32            5 mm F16
+    //   160x120     62 /  67 /  74      75 /  82 /  91
+    //   262x196     65 /  69 /  74      73 /  78 /  83
+    //   283x212     70 /  70 /  78      75 /  75 /  81
+    //   320x240     72 /  70 /  75      78 /  79 /  86
+    //   413x310     89 /  80 /  81      97 /  85 /  89
+    //   462x346     99 /  81 /  78     109 /  87 /  88
+    //   516x387    112 /  88 /  79     124 /  93 /  93
+    //   640x480    142 / 103 /  86     164 / 116 /  98
+    // The lines lie where neither side is better.  Marches of several sessions fill
+    // the GPU beside one another and take full warps.
+    const long long px = (long long)cam.w * cam.h;
+    if (px <= 60000 && !shared)
         launch_march_rays<WX, WY, 8>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, dependent);
     else if (px <= 160000 && !shared)
         launch_march_rays<WX, WY, 16>(m, fmt, cam, P, rb, vmap, vmap_pitch_elems, skip, s, dependent);
