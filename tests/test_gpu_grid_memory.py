@@ -4,6 +4,8 @@ the hash table, the same bits."""
 from __future__ import annotations
 
 import gc
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -85,3 +87,41 @@ def test_no_session_is_refused_for_its_grid(cuda, sessions):
             r = sorted(tight.poll(), key=lambda r: r["session"])
             assert np.array_equal(r[0]["Tcm"], want[k + 2][0]) and np.array_equal(r[1]["Tcm"], want[k][1])
     tight.close()
+
+
+def test_a_busy_session_gives_its_grid_back(cuda):
+    """Its queue does not empty while another session is opened: that one waits for a
+    frame, not for the queue."""
+    w, h, kw = 160, 120, dict(hash_slots=1 << 20, max_blocks=1 << 17, voxel_size=0.004, num_levels=3)
+    seq, K = sequence(7, 4, w, h), synth.intrinsics(w, h)
+    need = _estimate(w, h, 3, 1 << 20, 1 << 17)
+    probe = serving.Server(hbm_reserve_bytes=1 << 30)
+    before = _free()
+    own = (probe.open(w, h, K, **kw), before - _free())[1]
+    probe.close()
+    srv = serving.Server(hbm_reserve_bytes=_free() - (own - 17 * MB) - need - 6 * MB)
+    first = srv.open(w, h, K, **kw)
+    walk = [0, 1, 2, 3, 2, 1]
+    stop, sent = threading.Event(), [0]
+
+    def feed():
+        while not stop.is_set():
+            if srv.submit(first, *seq[walk[sent[0] % 6]][:2]) == 0:
+                sent[0] += 1
+
+    t = threading.Thread(target=feed)
+    t.start()
+    try:
+        while sent[0] < 200:
+            time.sleep(0.001)
+        since = time.monotonic()
+        second = srv.open(w, h, K, **kw)
+        took = time.monotonic() - since
+    finally:
+        stop.set()
+        t.join()
+    assert took < 5.0
+    assert srv.submit(second, *seq[0][:2]) == 0
+    srv.drain()
+    assert sum(r["session"] == first and r["status"] == 0 for r in srv.poll(1 << 16)) == sent[0]
+    srv.close()

@@ -78,6 +78,7 @@ struct ServedSession {
     bool gn_running = false;      // its share counts against the co-resident CTAs
     long long submitted = 0, completed = 0;
     bool closing = false;
+    bool held = false;       // starts no frame for the moment (its block grid is being given back)
     bool suspended = false;  // map swapped out to host memory; frames wait in the queue
 };
 
@@ -300,7 +301,7 @@ void worker_main(yas_server *srv) {
         // every session with a queued frame and none in flight starts it now
         for (ServedSession *ss : srv->sessions) {
             if (!ss) continue;
-            if (!ss->closing && !ss->suspended && !ss->in_flight && !ss->queue.empty() && st == YAS_OK) {
+            if (!ss->closing && !ss->suspended && !ss->held && !ss->in_flight && !ss->queue.empty() && st == YAS_OK) {
                 st = session_needs_init(ss->s) ? launch_first(ss) : launch_pre_frame(ss);
                 if (st == YAS_OK && ss->awaiting_gn && srv->cfg.gn_per_session) srv->own_wait.push_back(ss);
                 launched = true;
@@ -396,11 +397,16 @@ static int free_memory(yas_server *srv, size_t need, size_t *out) {
     {
         std::unique_lock<std::mutex> lk(srv->mu);
         for (size_t i = 0; i < srv->sessions.size(); ++i) {
-            // (the worker starts a frame with the lock held)
-            srv->cv.wait(lk, [&] { return !srv->sessions[i] || !srv->sessions[i]->in_flight || srv->stop.load(); });
-            if (srv->sessions[i] && !srv->sessions[i]->in_flight) session_drop_grid(srv->sessions[i]->s);
+            ServedSession *ss = srv->sessions[i];
+            if (!ss) continue;
+            ss->held = true;  // or a queue that never empties would keep it in flight
+            srv->cv.wait(lk, [&] { return srv->sessions[i] != ss || !ss->in_flight || srv->stop.load(); });
+            if (srv->sessions[i] != ss) continue;  // closed meanwhile
+            if (!ss->in_flight) session_drop_grid(ss->s);
+            ss->held = false;
         }
     }
+    srv->cv.notify_all();
     YAS_TRY_CUDA(cudaMemGetInfo(out, &total));
     return YAS_OK;
 }
