@@ -257,12 +257,13 @@ __device__ __forceinline__ int2 nearest_pixel2(float2 s, float2 &off) {
 // observation removed again (de-integration, for re-integration after a pose
 // correction): s <- (s w - d) / (w - 1), w <- w - 1; exact while the weight
 // stayed below the cap, as the reference's running average is then invertible.
-// Bound by instruction issue (the depth image and the blocks are in L2): a
-// thread projects its four voxels two at a time with packed FP32, starts their
-// depth reads, and then updates all four under one branch.  13 k visible blocks
-// at 640x480, 5 mm F16: 37.8 -> 25.6 us (80 % of the issue slots; before, a
-// correctly rounded reciprocal, conversions and a branch per voxel), 1280x720,
-// 4 mm F16: 59.8 -> 39.7, 320x240, 8 mm F32: 15.7 -> 12.6.
+// Bound by instruction issue and by the latency of its reads (the depth image and
+// the blocks are in L2): a thread projects its four voxels two at a time with
+// packed FP32, starts their depth reads, and then updates all four under one
+// branch.  13 k visible blocks at 640x480, 5 mm F16: 37.8 -> 25.6 us (before, a
+// correctly rounded reciprocal, conversions and a branch per voxel; now 16.2 M warp
+// instructions for 30.9 M, 65 % of the issue slots for 75 %, 29 warps an SM),
+// 1280x720, 4 mm F16: 59.8 -> 39.7, 320x240, 8 mm F32: 15.7 -> 12.6.
 template <int FMT, int SIGN>
 __global__ void __launch_bounds__(256) integrate_kernel(MapDev m, const float *__restrict__ depth,
                                                         int pitch, Cam cam, const PosePair *P,

@@ -24,7 +24,7 @@
 // cross the layers that drift left (at 640x480, 5 mm after 1000 frames 38
 // samples a ray instead of 11, 10 of them interpolated).  There the warps are
 // bound by the instructions of an iteration, whose lanes look up, jump and
-// interpolate in turn (14 of 32 active, 65% of the issue slots), and the last by
+// interpolate in turn (14 of 32 active, 63% of the issue slots), and the last by
 // the chain of the longest rays; floors without conversion instructions, the
 // neighbours of a cell read side by side, and packed lerps take such a raycast
 // (its other kernels included) from 264 to 218 us, a new map's from 115 to 109,
