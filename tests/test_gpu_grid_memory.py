@@ -12,6 +12,7 @@ import pytest
 import torch
 
 from tests.helpers import sequence
+from yetanotherslam_gb300 import _lib as L
 from yetanotherslam_gb300 import rgbdfusion as rf
 from yetanotherslam_gb300 import serving, synth
 
@@ -124,4 +125,14 @@ def test_a_busy_session_gives_its_grid_back(cuda):
     assert srv.submit(second, *seq[0][:2]) == 0
     srv.drain()
     assert sum(r["session"] == first and r["status"] == 0 for r in srv.poll(1 << 16)) == sent[0]
+    srv.close()
+
+
+def test_a_session_that_cannot_fit_costs_nobody_a_grid(cuda):
+    srv = serving.Server(hbm_reserve_bytes=1 << 30)
+    srv.open(160, 120, synth.intrinsics(160, 120), hash_slots=1 << 16, max_blocks=1 << 12, voxel_size=0.01)
+    before = _free()
+    with pytest.raises(L.YasError):
+        srv.open(160, 120, synth.intrinsics(160, 120), hash_slots=1 << 20, max_blocks=1 << 29, voxel_size=0.01)
+    assert _free() == before
     srv.close()

@@ -389,16 +389,20 @@ YAS_API int yas_server_create(yas_server **out, const yas_server_config *cfg) {
 }
 
 // Free device memory, at least `need` of it if that is to be had: where it is short
-// the sessions' block grids go first, so that they make nobody wait or be refused.
+// the sessions' block grids go first, so that nobody is refused for them (and stay
+// where they would not be enough).
 static int free_memory(yas_server *srv, size_t need, size_t *out) {
     size_t total = 0;
     YAS_TRY_CUDA(cudaMemGetInfo(out, &total));
     if (*out >= need) return YAS_OK;
     {
         std::unique_lock<std::mutex> lk(srv->mu);
+        size_t grids = 0;
+        for (ServedSession *ss : srv->sessions) grids += ss && session_has_grid(ss->s) ? kGridBytes : 0;
+        if (*out + grids < need) return YAS_OK;
         for (size_t i = 0; i < srv->sessions.size(); ++i) {
             ServedSession *ss = srv->sessions[i];
-            if (!ss) continue;
+            if (!ss || !session_has_grid(ss->s)) continue;
             ss->held = true;  // or a queue that never empties would keep it in flight
             srv->cv.wait(lk, [&] { return srv->sessions[i] != ss || !ss->in_flight || srv->stop.load(); });
             if (srv->sessions[i] != ss) continue;  // closed meanwhile

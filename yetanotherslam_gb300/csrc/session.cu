@@ -488,7 +488,7 @@ static int refresh_grid(yas_session *s) {
     const unsigned long long additions = s->map->additions;
     if (additions == s->grid_additions) return YAS_OK;
     s->grid_additions = additions;
-    if (s->frames == 0) return YAS_OK;  // the initialising frame does not raycast
+    if (s->frames == 0 || !s->zt.grid.cells) return YAS_OK;  // (the initialising frame does not raycast)
     launch_block_grid(map_view(s->map), &s->fs->pp, s->zt, s->stream);
     YAS_TRY_CUDA(cudaGetLastError());
     return YAS_OK;
@@ -624,8 +624,10 @@ YAS_API int yas_session_destroy(yas_session *s);
 
 namespace yas {
 
+bool session_has_grid(const yas_session *s) { return s->zt.grid.cells != nullptr; }
+
 void session_drop_grid(yas_session *s) {
-    if (!s->zt.grid.cells) return;
+    if (!session_has_grid(s)) return;
     cudaStreamSynchronize(s->stream);
     drop_graphs(s);  // they name the cells
     block_grid_free(s->zt.grid);

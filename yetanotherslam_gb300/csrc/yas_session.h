@@ -23,6 +23,7 @@ struct LaunchShape {
 // yas_session_create for arguments that were looked at; without its block grid, the
 // session's raycasts look blocks up in the hash table (the same results, slower).
 int session_create(yas_session **out, const yas_session_config *cfg, void *stream, bool block_grid);
+bool session_has_grid(const yas_session *s);
 // Gives the block grid's memory back (no frame of the session may be in flight).
 void session_drop_grid(yas_session *s);
 // Copies one frame (RGB u8 interleaved, depth u16) into the session's device
